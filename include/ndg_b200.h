@@ -251,9 +251,9 @@ ndg_status ndg_adapt_flags(ndg_ctx* ctx, const int32_t* refine, const double* p_
  * *avg_ms = mean kernel duration. */
 ndg_status ndg_time_stage(ndg_ctx* ctx, int32_t m, int32_t n_launches, double* avg_ms);
 
-/* Autotuner (no reference counterpart). The uniform-order stage kernel is
+/* Autotuner (no reference counterpart). The uniform-order stage kernels are
  * compiled for several tiles (elements per CTA: 2, 4, 8, 16 where a tile
- * fits 512 threads and 113 KB of shared memory) besides its default.
+ * fits 512 threads and an SM's shared memory) besides their default.
  * ndg_autotune times n_launches launches of each tile, and of the default,
  * on the loaded mesh and instances in the context's current form (FP64 or
  * FP32), keeps the fastest for later stepping and returns it (0 = the
@@ -264,7 +264,10 @@ ndg_status ndg_time_stage(ndg_ctx* ctx, int32_t m, int32_t n_launches, double* a
 ndg_status ndg_autotune(ndg_ctx* ctx, int32_t n_launches, int32_t* elements_per_block, double* best_ms);
 /* Sets the tile of the current form by hand (0 = the default). */
 ndg_status ndg_set_tile(ndg_ctx* ctx, int32_t elements_per_block);
-/* The candidate tiles of the loaded order and current form, and the default. */
+/* The candidate tiles of the loaded order and current form, and the default
+ * tile of the kernel with three threads per element line (the one that runs
+ * with ndg_ctx_keep_derivative). The kernel with one thread per line, which
+ * runs most orders, has a default of its own: 16 elements up to order 10. */
 ndg_status ndg_tile_candidates(const ndg_ctx* ctx, int32_t* out, int32_t capacity, int32_t* count, int32_t* default_tile);
 
 /* No counterpart in the reference. Host wall time of the last adaptation

@@ -193,13 +193,30 @@ cudaError_t issue_general_stage(ndg_ctx* c, int m, int in) {
     return err;
 }
 
+// Whether the uniform stage runs the line kernel (line_stage.cuh): on a mesh
+// of its orders and sizes, in the default and FP32 forms, with its own tiles.
+// The time derivative (keep_derivative) is a by-product only of the
+// three-threads-a-line kernel, which also runs where a periodic seam's two
+// normals are not opposite.
+bool line_mesh(const ndg_ctx* c) { return !c->general && c->seams_opposite && dev::line_kernel_runs(c->N, fp32(c), c->K * c->n_instances); }
+bool line_stage(const ndg_ctx* c) {
+    return line_mesh(c) && !strict(c) && !c->keep_derivative && c->tile[fp32(c) ? 1 : 0] < dev::kTensorTile;
+}
+// Whether the tile codes below kTensorTile are the line kernel's.
+bool line_tiles(const ndg_ctx* c) { return line_mesh(c) || dev::line_kernel_always(c->N); }
+
 cudaError_t issue_stage(ndg_ctx* c, int m, int in) {
     if (c->general) return issue_general_stage(c, m, in);
+    if (line_stage(c))
+        return fp32(c) ? dev::launch_line_fp32(c->N, c->tile[1], stage_args(c, m, in), c->stream)
+                       : dev::launch_line_fp64(c->N, c->tile[0], stage_args(c, m, in), c->stream);
+    const int tile = c->tile[fp32(c) ? 1 : 0];
+    const bool variant = tile >= dev::kTensorTile || !line_tiles(c);
     if (fp32(c)) {
-        if (c->tile[1]) return dev::launch_stage_variant_fp32(c->N, c->tile[1], stage_args(c, m, in), c->stream);
+        if (tile && variant) return dev::launch_stage_variant_fp32(c->N, c->tile[1], stage_args(c, m, in), c->stream);
         return dev::launch_stage_f32(c->N, stage_args(c, m, in), c->stream);
     }
-    if (!strict(c) && c->tile[0]) return dev::launch_stage_variant_fp64(c->N, c->tile[0], stage_args(c, m, in), c->stream);
+    if (!strict(c) && tile && variant) return dev::launch_stage_variant_fp64(c->N, c->tile[0], stage_args(c, m, in), c->stream);
     return dev::launch_stage(c->N, strict(c), stage_args(c, m, in), c->stream);
 }
 
@@ -232,7 +249,7 @@ void launch_stage(ndg_ctx* c, int m) {
 // The tile candidates of the context's form (FP64 or FP32).
 std::vector<int> tile_candidates(const ndg_ctx* c) {
     int buf[16];
-    const int n = fp32(c) ? dev::tile_candidates_fp32(c->N, buf, 16) : dev::tile_candidates_fp64(c->N, buf, 16);
+    const int n = fp32(c) ? dev::tile_candidates_fp32(c->N, line_tiles(c), buf, 16) : dev::tile_candidates_fp64(c->N, line_tiles(c), buf, 16);
     return std::vector<int>(buf, buf + n);
 }
 
@@ -240,14 +257,16 @@ void set_tile(ndg_ctx* c, int epb) {
     if (epb != 0) {
         const std::vector<int> cand = tile_candidates(c);
         if (std::find(cand.begin(), cand.end(), epb) == cand.end()) fail(NDG_ERR_INVALID_ARG, "not a candidate tile of this order and form");
-        check_cuda(fp32(c) ? dev::prepare_stage_variant_fp32(c->N, epb) : dev::prepare_stage_variant_fp64(c->N, epb), "kernel attributes");
+        check_cuda(fp32(c) ? dev::prepare_stage_variant_fp32(c->N, line_tiles(c), epb) : dev::prepare_stage_variant_fp64(c->N, line_tiles(c), epb), "kernel attributes");
     }
     c->tile[fp32(c) ? 1 : 0] = epb;
     drop_graphs(c);
 }
 
 void ensure_traces(ndg_ctx* c) {
-    if (c->traces_valid) return;
+    const bool line = line_stage(c);
+    if (c->traces_valid && c->line_traces == line) return;
+    c->line_traces = line;
     if (c->general) {
         require_form(c);
         dev::GeneralStage g = general_args(c, 0, c->cur);
@@ -261,6 +280,7 @@ void ensure_traces(ndg_ctx* c) {
     a.q = c->q.ptr;
     a.trace_out = c->tr[c->cur].ptr;
     a.link = reinterpret_cast<const int2*>(c->link.ptr);  // far-slot layout of the stage kernels
+    a.normal = reinterpret_cast<const double2*>(c->normal.ptr);
     a.n_elements = c->K;
     a.field_stride = c->Kp;
     a.n_instances = c->n_instances;
@@ -271,7 +291,10 @@ void ensure_traces(ndg_ctx* c) {
             if (t.count != count) t.allocate(count);
         a.trace_out_f = c->tr32[c->cur].ptr;
         check_cuda(dev::prepare_kernels_f32(c->N), "kernel attributes");
-        check_cuda(dev::launch_traces_f32(c->N, a, c->stream), "trace kernel launch");
+        if (line) check_cuda(dev::prepare_line_fp32(c->N, 0), "kernel attributes");
+        check_cuda(line ? dev::launch_line_traces_fp32(c->N, a, c->stream) : dev::launch_traces_f32(c->N, a, c->stream), "trace kernel launch");
+    } else if (line) {
+        check_cuda(dev::launch_line_traces_fp64(c->N, a, c->stream), "trace kernel launch");
     } else {
         check_cuda(dev::launch_traces(c->N, strict(c), a, c->stream), "trace kernel launch");
     }
@@ -386,6 +409,17 @@ void upload_plan(ndg_ctx* c, const Layout& l) {
     if (!l.general) {
         if (c->N > kMaxOrder) fail(NDG_ERR_UNSUPPORTED, "orders above 16 have no compiled kernel");
         SidePlan plan = build_side_plan(c->topo, c->tables);
+        // Outward normals n of the two sides of an interior link: opposite to
+        // rounding on every conforming face and on seams that are translates.
+        c->seams_opposite = true;
+        for (size_t i = 0; i < 4 * K && c->seams_opposite; ++i) {
+            const int32_t word = plan.link[2 * i + 1];
+            if (((word >> 2) & 7) != kInterior) continue;
+            const size_t o = 4 * static_cast<size_t>(plan.link[2 * i]) + static_cast<size_t>(word & 3);
+            const double s = ((word >> 5) & 1) == ((plan.link[2 * o + 1] >> 5) & 1) ? 1.0 : -1.0;
+            for (size_t d = 0; d < 2; ++d)
+                if (std::abs(plan.normal[2 * i + d] + s * plan.normal[2 * o + d]) > 1e-15) c->seams_opposite = false;
+        }
         // Tiles copy an even number of elements: pad the per-element arrays
         // to the even element count (the pad element has no sides).
         const size_t Kpad = static_cast<size_t>(c->Kp);
@@ -408,6 +442,7 @@ void upload_plan(ndg_ctx* c, const Layout& l) {
         c->tc32.upload(dev::tc_lane_table_fp32(c->N), c->stream);
         check_cuda(dev::prepare_kernels(c->N, false), "kernel attributes");
         check_cuda(dev::prepare_kernels(c->N, true), "kernel attributes");
+        if (dev::line_kernel_runs(c->N, false, c->K * c->n_instances)) check_cuda(dev::prepare_line_fp64(c->N, 0), "kernel attributes");
         c->groups.clear();
         c->whole_groups.clear();
     } else {

@@ -51,6 +51,7 @@ struct TraceArgs {
     int64_t field_stride;
     int n_instances;
     const int2* link = nullptr;
+    const double2* normal = nullptr;  // line kernel
 };
 
 cudaError_t prepare_kernels(int N, bool strict);
@@ -72,12 +73,26 @@ int elements_per_block(int N);
 // Candidate tiles of the autotuner (stage_variants_fp64.cu, _fp32.cu): the
 // feasible elements-per-CTA values of order N, and the stage kernel with
 // one of them (FP64 default rounding, or the FP32 form).
-int tile_candidates_fp64(int N, int* out, int max);
-int tile_candidates_fp32(int N, int* out, int max);
-cudaError_t prepare_stage_variant_fp64(int N, int epb);
-cudaError_t prepare_stage_variant_fp32(int N, int epb);
+int tile_candidates_fp64(int N, bool line, int* out, int max);  // line: the line kernel's tiles
+int tile_candidates_fp32(int N, bool line, int* out, int max);
+cudaError_t prepare_stage_variant_fp64(int N, bool line, int epb);
+cudaError_t prepare_stage_variant_fp32(int N, bool line, int epb);
 cudaError_t launch_stage_variant_fp64(int N, int epb, const StageArgs& a, cudaStream_t stream);
 cudaError_t launch_stage_variant_fp32(int N, int epb, const StageArgs& a, cudaStream_t stream);
+// The line kernel (line_stage.cuh; elements = 0: its default tile): whether it
+// runs order N, its candidate tiles, and its first traces. Its traces are one
+// outgoing characteristic per side node, [instance][field_stride][side][N+1]
+// in the far slots, at the start of the trace buffers.
+bool line_kernel_runs(int N, bool fp32, int64_t elements);  // elements of all instances
+bool line_kernel_always(int N);                             // at every size: no three-threads-a-line tiles are compiled
+int line_candidates_fp64(int N, int* out, int max);
+int line_candidates_fp32(int N, int* out, int max);
+cudaError_t prepare_line_fp64(int N, int elements);
+cudaError_t prepare_line_fp32(int N, int elements);
+cudaError_t launch_line_fp64(int N, int elements, const StageArgs& a, cudaStream_t stream);
+cudaError_t launch_line_fp32(int N, int elements, const StageArgs& a, cudaStream_t stream);
+cudaError_t launch_line_traces_fp64(int N, const TraceArgs& a, cudaStream_t stream);
+cudaError_t launch_line_traces_fp32(int N, const TraceArgs& a, cudaStream_t stream);
 // Tile codes at or above kTensorTile select the tensor-core contraction
 // variant with (code - kTensorTile) elements per CTA.
 constexpr int kTensorTile = 100;

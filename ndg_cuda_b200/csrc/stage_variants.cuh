@@ -4,9 +4,11 @@
 // free layout needs) where the tile fits 512 threads and 113 KB of shared
 // memory (two CTAs per SM).
 // stage_variants_fp64.cu and stage_variants_fp32.cu instantiate these
-// templates for the FP64 (default rounding) and the FP32 form.
+// templates for the FP64 (default rounding) and the FP32 form; where the line
+// kernel runs, the candidates are its tiles (line_stage.cuh).
 #pragma once
 
+#include "line_stage.cuh"
 #include "stage_templates.cuh"
 
 #include <cuda_runtime.h>
@@ -25,7 +27,8 @@ constexpr int kTensorMinOrder = 6;
 template <bool F32, int N, int E, bool TC = false>
 struct Variant {
     using T = std::conditional_t<F32, TileF<N, E>, Tile<N, E>>;
-    static constexpr bool feasible = T::kThreads <= 512 && T::kBytes <= 113 * 1024 && (!TC || (E <= 8 && N >= kTensorMinOrder));
+    // Orders that run the line kernel at every size have no SIMT tiles.
+    static constexpr bool feasible = T::kThreads <= 512 && T::kBytes <= 113 * 1024 && (TC ? E <= 8 && N >= kTensorMinOrder : !line_every_size(N));
 };
 
 template <int N>

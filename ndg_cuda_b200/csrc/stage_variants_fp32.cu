@@ -19,13 +19,14 @@ int simt_candidates(int N, int* out, int max) {
 }
 }  // namespace
 
-int tile_candidates_fp32(int N, int* out, int max) {
-    const int c = simt_candidates(N, out, max);
+int tile_candidates_fp32(int N, bool line, int* out, int max) {
+    const int c = line ? line_candidates_fp32(N, out, max) : simt_candidates(N, out, max);
     return c + tile_candidates_tc32(N, out + c, max - c);
 }
 
-cudaError_t prepare_stage_variant_fp32(int N, int epb) {
+cudaError_t prepare_stage_variant_fp32(int N, bool line, int epb) {
     if (epb >= kTensorTile) return prepare_stage_variant_tc32(N, epb - kTensorTile);
+    if (line) return prepare_line_fp32(N, epb);
 #define NDG_CALL(n) return variant_prepare_n<true, n, false>(epb)
     NDG_VARIANT_ORDERS(NDG_CALL)
 #undef NDG_CALL

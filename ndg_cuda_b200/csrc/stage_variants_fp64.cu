@@ -19,13 +19,14 @@ int simt_candidates(int N, int* out, int max) {
 }
 }  // namespace
 
-int tile_candidates_fp64(int N, int* out, int max) {
-    const int c = simt_candidates(N, out, max);
+int tile_candidates_fp64(int N, bool line, int* out, int max) {
+    const int c = line ? line_candidates_fp64(N, out, max) : simt_candidates(N, out, max);
     return c + tile_candidates_tc64(N, out + c, max - c);
 }
 
-cudaError_t prepare_stage_variant_fp64(int N, int epb) {
+cudaError_t prepare_stage_variant_fp64(int N, bool line, int epb) {
     if (epb >= kTensorTile) return prepare_stage_variant_tc64(N, epb - kTensorTile);
+    if (line) return prepare_line_fp64(N, epb);
 #define NDG_CALL(n) return variant_prepare_n<false, n, false>(epb)
     NDG_VARIANT_ORDERS(NDG_CALL)
 #undef NDG_CALL

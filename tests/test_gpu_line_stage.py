@@ -1,0 +1,97 @@
+"""The uniform stage kernel with one thread per element line, against the
+three-threads-a-line kernel (which keep_derivative selects) and the oracle.
+
+Sizes are the edges of its dispatch and tiles: element counts just below and
+above the size rule (1,536 elements times the instances), ragged last tiles,
+odd counts, every order it runs, every boundary kind, one and several
+instances. Both kernels evaluate the same operator in FP64 (or the FP32
+form's FP32 part), so the difference after a few steps is rounding: with
+n + 1 = N + 2 term sums and a dozen operations per stage, 1e-13 relative L2
+leaves a factor of ten over FP64's 2^-53 times the terms and stages; the FP32
+form is held to its own 1e-6 of FP64 on either side, 2e-6 between them.
+"""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import ndg_cuda_b200 as ndg
+from oracle.pyoracle import OracleSolver
+from tests import meshgen
+
+pytestmark = pytest.mark.gpu
+
+
+def rel_l2(a, b):
+    return float(np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-300))
+
+
+def _run(zone, N, precision, keep, fields, n_inst, steps, tiles=(0,)):
+    m = ndg.Mesh2D_t(zone, N, precision=precision, n_instances=n_inst, keep_derivative=keep)
+    out = []
+    for tile in tiles:
+        m.set_tile(tile)
+        for f, v in zip(("p", "u", "v"), fields):
+            m.set_field(f, v)
+        ndg.Solver2D_t.run(m, steps)
+        out.append(np.concatenate([m.get_field(f) for f in ("p", "u", "v", "k_p", "k_u", "k_v")]))
+    m.close()
+    return out
+
+
+CASES = [("periodic", 40, 1, 0.1), ("wall", 41, 1, 0.1), ("outflow", 20, 4, 0.0), ("inflow", 39, 1, 0.1)]
+
+
+@pytest.mark.parametrize("precision", [ndg.FP64, ndg.FP32])
+@pytest.mark.parametrize("N", list(range(1, 15)))
+@pytest.mark.parametrize("kind,res,n_inst,jitter", CASES)
+def test_line_kernel_against_three_threads_a_line(N, precision, kind, res, n_inst, jitter):
+    kw = {"periodic": dict(x_periodic=True, y_periodic=True), "wall": dict(x_periodic=True, boundary=meshgen.WALL),
+          "outflow": dict(boundary=meshgen.OUTFLOW), "inflow": dict(boundary=meshgen.INFLOW, x_min=0.0, x_max=1.0, y_min=0.0, y_max=1.0)}[kind]
+    zone = meshgen.uniform_zone(res, order="rowmajor", jitter=jitter, seed=res, **kw)
+    rng = np.random.default_rng(N)
+    K = res * res
+    fields = [rng.standard_normal(n_inst * K * (N + 1) ** 2) for _ in range(3)]
+    line, = _run(zone, N, precision, False, fields, n_inst, 2)
+    three, = _run(zone, N, precision, True, fields, n_inst, 2)
+    assert rel_l2(line, three) < (1e-13 if precision == ndg.FP64 else 2e-6)
+
+
+@pytest.mark.parametrize("precision", [ndg.FP64, ndg.FP32])
+@pytest.mark.parametrize("N", [7, 8, 11])
+def test_line_tiles_agree_and_runs_split_anywhere(N, precision):
+    """Tiles give the same bits, and so does a run stopped and resumed after
+    its traces were rebuilt from q."""
+    zone = meshgen.uniform_zone(40, order="rowmajor", x_periodic=True, boundary=meshgen.WALL, jitter=0.1, seed=3)
+    m = ndg.Mesh2D_t(zone, N, precision=precision)
+    tiles = [0] + [t for t in m.tile_candidates()[0] if t < ndg.TENSOR_TILE]
+    rng = np.random.default_rng(0)
+    fields = [rng.standard_normal(m.field_size) for _ in range(3)]
+    m.close()
+    runs = _run(zone, N, precision, False, fields, 1, 4, tiles)
+    for t, r in zip(tiles[1:], runs[1:]):
+        assert np.array_equal(r, runs[0]), t
+    m = ndg.Mesh2D_t(zone, N, precision=precision)
+    for f, v in zip(("p", "u", "v"), fields):
+        m.set_field(f, v)
+    ndg.Solver2D_t.run(m, 2)
+    m.set_field("u", m.get_field("u"))
+    ndg.Solver2D_t.run(m, 2)
+    got = np.concatenate([m.get_field(f) for f in ("p", "u", "v", "k_p", "k_u", "k_v")])
+    m.close()
+    assert np.array_equal(got, runs[0])
+
+
+@pytest.mark.parametrize("N", [5, 8])
+def test_line_kernel_against_the_oracle(N):
+    zone = meshgen.uniform_zone(40, order="rowmajor", boundary=meshgen.WALL, jitter=0.1, seed=5)
+    o = OracleSolver(zone, N)
+    o.initial_conditions()
+    m = ndg.Mesh2D_t(zone, N)
+    for f in ("p", "u", "v"):
+        m.set_field(f, o.field(f))
+    o.run(4)
+    ndg.Solver2D_t.run(m, 4)
+    for f in ("p", "u", "v"):
+        assert rel_l2(m.get_field(f), o.field(f)) < 1e-12, f
+    m.close()
