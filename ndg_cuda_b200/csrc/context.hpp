@@ -159,7 +159,9 @@ struct ndg_ctx {
     // run concurrently (forked from and joined to `stream`).
     std::vector<cudaStream_t> aux_streams;
     std::vector<cudaEvent_t> aux_events;
+    // Graphs by trace-buffer parity: one step, and kGraphSteps steps.
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
+    cudaGraphExec_t graph_many[2] = {nullptr, nullptr};
     int64_t launches = 0;
     // Incremented whenever the topology or its device plan changes (load,
     // adaptation): objects built on the mesh (adjoint problems) check it.
@@ -170,6 +172,8 @@ struct ndg_ctx {
 
     ~ndg_ctx() {
         for (auto& g : graph)
+            if (g) cudaGraphExecDestroy(g);
+        for (auto& g : graph_many)
             if (g) cudaGraphExecDestroy(g);
         for (auto& e : aux_events) cudaEventDestroy(e);
         for (auto& st : aux_streams) cudaStreamDestroy(st);

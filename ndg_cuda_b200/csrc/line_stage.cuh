@@ -322,6 +322,38 @@ __global__ void __launch_bounds__(LineTile<N, R, E>::kThreads, LineTile<N, R, E>
         if (tid == 0) {
             mbar_init(bar, 1);
             mbar_fence_init();
+        }
+    }
+    // Side data of the mesh plan, thread (element, side) with the side fastest.
+    // The first of a thread's are read ahead of the wait for the launch before
+    // and kept in registers until the tile's copies are on their way.
+    struct SidePlanEntry {
+        int2 lk;
+        double2 nv, c0, c1;
+    };
+    const auto read_side = [&](int i) {
+        const int64_t o = 4 * e0 + i;
+        return SidePlanEntry{a.link[o], a.normal[o], reinterpret_cast<const double2*>(a.corners)[o],
+                             reinterpret_cast<const double2*>(a.corners)[(o & ~int64_t{3}) + ((i + 1) & 3)]};
+    };
+    const auto put_side = [&](int i, const SidePlanEntry& p) {
+        const bool role = (p.lk.y >> 5) & 1;
+        const int kind = (p.lk.y >> 2) & 7;
+        const R dx = R(p.c1.x - p.c0.x), dy = R(p.c1.y - p.c0.y);
+        const int o = (i & 3) * E + (i >> 2);
+        side[o] = R(role ? -p.nv.x : p.nv.x);
+        side[4 * E + o] = R(role ? -p.nv.y : p.nv.y);
+        side[8 * E + o] = R(0.5) * sqrt(dx * dx + dy * dy);
+        side[12 * E + o] = dx;
+        side[16 * E + o] = dy;
+        to_s[o] = kind == kInterior ? (p.lk.x * 4 + (p.lk.y & 3)) : ~kind;
+    };
+    SidePlanEntry first_side{};
+    if (tid < 4 * ne) first_side = read_side(tid);
+    pdl_wait();
+    if (a.step_next && blockIdx.x == 0 && blockIdx.y == 0 && tid == 0) advance_step(a.step, a.step_next);
+    if constexpr (T::kBulk) {
+        if (tid == 0) {
             const uint32_t bytes = static_cast<uint32_t>(((ne + 1) & ~1) * NN * sizeof(double));
             mbar_expect_tx(bar, (a.first ? 3 : 6) * bytes);
             for (int f = 0; f < 3; ++f) bulk_load(qs + f * QS, q + (f * Kp + e0) * NN, bytes, bar);
@@ -349,26 +381,8 @@ __global__ void __launch_bounds__(LineTile<N, R, E>::kThreads, LineTile<N, R, E>
         else
             cp_async4(far_s + el * SE + o, tr_in + (e0 + el) * 4 * n + o);
     }
-    // Side data, thread (element, side) with the side fastest.
-    for (int i = tid; i < 4 * E; i += T::kThreads) {
-        const int el = i >> 2, s = i & 3;
-        if (el < ne) {
-            const int2 lk = a.link[4 * (e0 + el) + s];
-            const double2 nv = a.normal[4 * (e0 + el) + s];
-            const double2 c0 = reinterpret_cast<const double2*>(a.corners)[4 * (e0 + el) + s];
-            const double2 c1 = reinterpret_cast<const double2*>(a.corners)[4 * (e0 + el) + ((s + 1) & 3)];
-            const bool role = (lk.y >> 5) & 1;
-            const int kind = (lk.y >> 2) & 7;
-            const R dx = R(c1.x - c0.x), dy = R(c1.y - c0.y);
-            const int o = s * E + el;
-            side[o] = R(role ? -nv.x : nv.x);
-            side[4 * E + o] = R(role ? -nv.y : nv.y);
-            side[8 * E + o] = R(0.5) * sqrt(dx * dx + dy * dy);
-            side[12 * E + o] = dx;
-            side[16 * E + o] = dy;
-            to_s[o] = kind == kInterior ? (lk.x * 4 + (lk.y & 3)) : ~kind;
-        }
-    }
+    if (tid < 4 * ne) put_side(tid, first_side);
+    for (int i = tid + T::kThreads; i < 4 * ne; i += T::kThreads) put_side(i, read_side(i));
     cp_async_wait_all();
     __syncthreads();
     if constexpr (T::kBulk) {
@@ -519,6 +533,7 @@ __global__ void __launch_bounds__(LineTile<N, R, E>::kThreads, LineTile<N, R, E>
     }
     if constexpr (T::kBulk) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
+    pdl_launch_dependents();
     if constexpr (T::kBulk) {
         if (tid == 0) {
             const uint32_t bytes = static_cast<uint32_t>(((ne + 1) & ~1) * NN * sizeof(double));

@@ -31,8 +31,7 @@ cudaError_t launch(const StageArgs& a, cudaStream_t stream) {
     if constexpr (usable<N, E>()) {
         using T = LineTile<N, R, E>;
         const dim3 grid(static_cast<unsigned>((a.n_elements + E - 1) / E), static_cast<unsigned>(a.n_instances));
-        line_stage_kernel<N, R, E><<<grid, T::kThreads, T::kBytes, stream>>>(a, make_line_coeffs<N, R>());
-        return cudaGetLastError();
+        return launch_dependent(line_stage_kernel<N, R, E>, grid, T::kThreads, T::kBytes, stream, a, make_line_coeffs<N, R>());
     } else {
         return cudaErrorInvalidValue;
     }

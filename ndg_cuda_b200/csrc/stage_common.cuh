@@ -170,6 +170,45 @@ __device__ __forceinline__ uint64_t evict_first_policy() {
 __device__ __forceinline__ void cp_async8_stream(void* dst, const void* src, uint64_t policy) {
     asm volatile("cp.async.ca.shared.global.L2::cache_hint [%0], [%1], 8, %2;" ::"r"(smem_addr(dst)), "l"(src), "l"(policy) : "memory");
 }
+// Programmatic dependent launch (PTX ISA: griddepcontrol). A kernel launched
+// by launch_dependent may start while the launch before it on the stream still
+// runs, once every CTA of that one has started (or called
+// pdl_launch_dependents). Before pdl_wait, which returns when the launches
+// before it are complete and their writes visible, it touches only its own
+// shared memory and arrays that no launch of the run writes (the mesh plan).
+// The stage kernels let the next launch start late, when their new state is
+// in shared memory: earlier, its CTAs crowd onto the SMs that happen to have
+// room and run unevenly (N = 14, 32 x 32: 9.3 us a stage late, 11.7 after the
+// tile's loads, 11.6 at the start; without overlap 10.4).
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename... Params, typename... Args>
+inline cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t stream, Args&&... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(static_cast<unsigned>(threads));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
+// Time update of the reference's loop (Solver2D_t.tcu:37-42, 72) with
+// step = {time, dt, dt_mesh, t_end}: advance, then the next step's dt,
+// shortened to land on t_end.
+__device__ __forceinline__ void advance_step(const double* step, double* next) {
+    const double time = step[0] + step[1];
+    next[0] = time;
+    next[1] = (time + step[2] > step[3]) ? step[3] - time : step[2];
+    next[2] = step[2];
+    next[3] = step[3];
+}
+
 // Hint: bring the 128-byte line holding p into L2 (prefetch.global.L2).
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 

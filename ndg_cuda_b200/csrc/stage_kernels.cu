@@ -191,13 +191,15 @@ __global__ void delta_t_kernel(const double* delta_xy_min, const int* elem_N, in
     if (threadIdx.x == 0) *out = red[0];
 }
 
-// Time update of the reference's loop (Solver2D_t.tcu:37-42, 72) with
-// step = {time, dt, dt_mesh, t_end}: advance, then the next step's dt,
-// shortened to land on t_end.
-__global__ void end_step_kernel(double* step) {
-    const double time = step[0] + step[1];
+// Time update at the end of a step on mixed-order meshes (the uniform stage
+// kernels do it themselves).
+__global__ void end_step_kernel(double* step) { advance_step(step, step); }
+
+__global__ void set_step_kernel(double* step, double time, double dt, double dt_mesh, double t_end) {
     step[0] = time;
-    step[1] = (time + step[2] > step[3]) ? step[3] - time : step[2];
+    step[1] = dt;
+    step[2] = dt_mesh;
+    step[3] = t_end;
 }
 
 // ---------------------------------------------------------------------------
@@ -314,8 +316,7 @@ template <int N, bool S>
 static cudaError_t launch_stage_t(const StageArgs& a, cudaStream_t stream) {
     using T = Tile<N>;
     const dim3 grid(static_cast<unsigned>((a.n_elements + T::EPB - 1) / T::EPB), static_cast<unsigned>(a.n_instances));
-    stage_kernel<N, S, 0><<<grid, T::kThreads, T::kBytes, stream>>>(a, make_coeffs<N>());
-    return cudaGetLastError();
+    return launch_dependent(stage_kernel<N, S, 0, false>, grid, T::kThreads, T::kBytes, stream, a, make_coeffs<N>());
 }
 
 template <int N, bool S>
@@ -385,8 +386,7 @@ template <int N, bool Unused>
 static cudaError_t launch_stage_f32_t(const StageArgs& a, cudaStream_t stream) {
     using T = TileF<N, 0>;
     const dim3 grid(static_cast<unsigned>((a.n_elements + T::EPB - 1) / T::EPB), static_cast<unsigned>(a.n_instances));
-    stage_kernel_f32<N, 0><<<grid, T::kThreads, T::kBytes, stream>>>(a, make_coeffs_f<N>());
-    return cudaGetLastError();
+    return launch_dependent(stage_kernel_f32<N, 0, false>, grid, T::kThreads, T::kBytes, stream, a, make_coeffs_f<N>());
 }
 
 template <int N, bool Unused>
@@ -446,6 +446,11 @@ cudaError_t launch_delta_t(const double* delta_xy_min, const int* elem_N, int64_
 
 cudaError_t launch_end_step(double* step, cudaStream_t stream) {
     end_step_kernel<<<1, 1, 0, stream>>>(step);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_set_step(double* step, double time, double dt, double dt_mesh, double t_end, cudaStream_t stream) {
+    set_step_kernel<<<1, 1, 0, stream>>>(step, time, dt, dt_mesh, t_end);
     return cudaGetLastError();
 }
 

@@ -29,6 +29,7 @@ struct StageArgs {
     const double* gscale;
     const double4* inflow;
     const double* step;  // {time, dt, dt_mesh, t_end}
+    double* step_next;   // last stage of a step: where the next step's goes (not `step`: all CTAs read that), else NULL
     unsigned* error;     // set when a bounded wait gives up
     const double* tc64;  // per-lane tables of the tensor-core passes (TcTable64 / TcTable32 of the order)
     const float* tc32;
@@ -65,6 +66,7 @@ cudaError_t launch_traces_f32(int N, const TraceArgs& a, cudaStream_t stream);
 cudaError_t launch_initial_conditions(double* q, double* k, const double* corners, int N, int64_t K, int64_t Kp, int n_instances, cudaStream_t stream);
 cudaError_t launch_delta_t(const double* delta_xy_min, const int* elem_N, int64_t K, double cfl, double* out, cudaStream_t stream);
 cudaError_t launch_end_step(double* step, cudaStream_t stream);
+cudaError_t launch_set_step(double* step, double time, double dt, double dt_mesh, double t_end, cudaStream_t stream);
 cudaError_t upload_tables(const Tables& t);
 // Host copy of the order-N coefficients uploaded by upload_tables: Dhat
 // ((N+1)^2), nodes, Lagrange values at -1 and +1, weights, 1/weights.

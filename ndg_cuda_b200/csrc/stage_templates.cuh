@@ -64,8 +64,10 @@ __global__ void __launch_bounds__(Tile<N, E>::kThreads, TC ? 0 : Tile<N, E>::kMi
     const double* xn = cf.xn;
     const double* lm = cf.lm;
     const double* lp = cf.lp;
+    pdl_wait();
     const double time = a.step[0];
     const double dt = a.step[1];
+    if (a.step_next && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) advance_step(a.step, a.step_next);
 
     // Line threads: (field f, line or node index m, element e of the tile),
     // e fastest (the order the bank-conflict-free strides assume).
@@ -475,6 +477,7 @@ __global__ void __launch_bounds__(Tile<N, E>::kThreads, TC ? 0 : Tile<N, E>::kMi
     }
     __syncthreads();
 
+    pdl_launch_dependents();
     // Side traces of the new solution for the next stage: bottom/top from
     // row m, right/left from column m (Element2D_t.cpp:86-125), written into
     // the far slots of the neighbour across each interior side (its side
@@ -600,8 +603,10 @@ __global__ void __launch_bounds__(TileF<N, E>::kThreads, TC ? 0 : TileF<N, E>::k
     const float* xn = cf.xn;
     const float* lm = cf.lm;
     const float* lp = cf.lp;
+    pdl_wait();
     const double time = a.step[0];
     const double dt = a.step[1];
+    if (a.step_next && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) advance_step(a.step, a.step_next);
 
     const int f = tid / (EPB * n);
     const int rr = tid - f * (EPB * n);
@@ -988,6 +993,7 @@ __global__ void __launch_bounds__(TileF<N, E>::kThreads, TC ? 0 : TileF<N, E>::k
     }
     __syncthreads();
 
+    pdl_launch_dependents();
     if (active) {
         const float* row = qf + f * QS + e * ES + m * P;
         const float* cl = qf + f * QS + e * ES + m;

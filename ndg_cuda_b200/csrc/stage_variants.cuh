@@ -74,10 +74,9 @@ cudaError_t variant_launch(const StageArgs& a, cudaStream_t stream) {
         using T = typename Variant<F32, N, E, TC>::T;
         const dim3 grid(static_cast<unsigned>((a.n_elements + T::EPB - 1) / T::EPB), static_cast<unsigned>(a.n_instances));
         if constexpr (F32)
-            stage_kernel_f32<N, E, TC><<<grid, T::kThreads, T::kBytes, stream>>>(a, variant_coeffs_f<N>());
+            return launch_dependent(stage_kernel_f32<N, E, TC>, grid, T::kThreads, T::kBytes, stream, a, variant_coeffs_f<N>());
         else
-            stage_kernel<N, false, E, TC><<<grid, T::kThreads, T::kBytes, stream>>>(a, variant_coeffs<N>());
-        return cudaGetLastError();
+            return launch_dependent(stage_kernel<N, false, E, TC>, grid, T::kThreads, T::kBytes, stream, a, variant_coeffs<N>());
     } else {
         return cudaErrorInvalidValue;
     }
