@@ -58,6 +58,7 @@ struct SpeedStageArgs {
     double rk_a, gdt;
     int first;
     int64_t n_elements, field_stride;
+    unsigned* error;  // set when a bounded wait gives up
     Receivers rec;
 };
 
@@ -89,8 +90,27 @@ struct AdjointStageArgs {
     Receivers rec;
 };
 
+// Pressure at the receivers of a tile, one warp: sum of w_r . p over the
+// element's nodes, lanes striding the nodes, then a shuffle reduction in a
+// fixed order (the same result wherever it is evaluated). FP64 in both forms.
+// Receiver sample sum_i w_i p_i over an element's nodes, with the element's
+// tile block p laid out in rows of pitch P (node i of n per row).
+template <int n, int P>
+__device__ __forceinline__ double receiver_value(const double* __restrict__ w, const double* p, int lane) {
+    double s = 0.0;
+    for (int i = lane; i < n * n; i += 32) s = fma(w[i], p[(i / n) * P + i % n], s);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+}
+
 cudaError_t prepare_speed_kernels(int N, bool fp32);
 cudaError_t launch_speed_stage(int N, bool fp32, const SpeedStageArgs& a, cudaStream_t stream);
+// The same stage by the line kernel (line_stage.cuh; where line_kernel_runs):
+// trace_in / trace_out then hold its characteristics (launch_line_traces_*),
+// and G_out is not written (with first set, k is G).
+cudaError_t prepare_speed_line(int N, bool fp32);
+cudaError_t launch_speed_line(int N, bool fp32, const SpeedStageArgs& a, cudaStream_t stream);
 cudaError_t launch_adjoint_stage(int N, bool fp32, const AdjointStageArgs& a, cudaStream_t stream);
 // grad_c[e] = acc[e][0] + sum over sides of acc[e][1+s] (boundary sides) or
 // (acc[e][1+s] + acc[nb][1+s']) / 2 (sides shared with element nb, side s').

@@ -36,6 +36,9 @@ struct ndg_adjoint {
     cudaEvent_t evr[2] = {nullptr, nullptr}, eva[2] = {nullptr, nullptr}, evs = nullptr;
     ndg::DeviceBuffer<float> tr_f[2], atr_f[2];  // traces of the FP32 form
     bool fp32 = false;
+    // The forward stage runs the line kernel in this form (by the rule of the
+    // uniform stage), with its characteristics in tr / tr_f.
+    bool line() const { return ctx->seams_opposite && ndg::dev::line_kernel_runs(N, fp32, K); }
     ndg::dev::Receivers rec{};
     // the last forward
     bool has_forward = false;
@@ -133,8 +136,13 @@ dev::SpeedStageArgs speed_args(ndg_adjoint* a, int m, int in, double dt) {
     s.first = m == 0;
     s.n_elements = a->K;
     s.field_stride = a->Kp;
+    s.error = c->error.ptr;
     s.rec = a->rec;
     return s;
+}
+
+cudaError_t launch_speed(ndg_adjoint* a, const dev::SpeedStageArgs& s, cudaStream_t stream) {
+    return a->line() ? dev::launch_speed_line(a->N, a->fp32, s, stream) : dev::launch_speed_stage(a->N, a->fp32, s, stream);
 }
 
 dev::AdjointStageArgs adjoint_args(ndg_adjoint* a, int in) {
@@ -167,7 +175,11 @@ void launch_traces_of_q(ndg_adjoint* a, int out, cudaStream_t stream = nullptr) 
     t.n_elements = a->K;
     t.field_stride = a->Kp;
     t.n_instances = 1;
-    if (a->fp32)
+    if (a->line()) {
+        t.link = reinterpret_cast<const int2*>(a->ctx->link.ptr);
+        t.normal = reinterpret_cast<const double2*>(a->ctx->normal.ptr);
+        check_cuda(a->fp32 ? dev::launch_line_traces_fp32(a->N, t, stream) : dev::launch_line_traces_fp64(a->N, t, stream), "trace kernel launch");
+    } else if (a->fp32)
         check_cuda(dev::launch_traces_f32(a->N, t, stream), "trace kernel launch");
     else
         check_cuda(dev::launch_traces(a->N, false, t, stream), "trace kernel launch");
@@ -177,6 +189,7 @@ void launch_traces_of_q(ndg_adjoint* a, int out, cudaStream_t stream = nullptr) 
 void check_kernel_error(ndg_adjoint* a) {
     check_cuda(cudaStreamSynchronize(a->ctx->stream), "adjoint-module kernels");
     check_cuda(cudaGetLastError(), "adjoint-module kernels");
+    check_device_error(a->ctx);
 }
 
 // Copies three host fields (field_size values each; NULL = zero) into a
@@ -208,7 +221,7 @@ int run_forward(ndg_adjoint* a, int in, int64_t first, int64_t last, double* q_s
             if (q_save) s.q_save = q_save + (static_cast<size_t>(step - first) * 3 + static_cast<size_t>(m)) * state;
             if (save_every > 0 && m == 0 && (step - 1) % save_every == 0) s.q_save = a->ckpt.ptr + static_cast<size_t>((step - 1) / save_every) * state;
             if (sample && m == 2 && a->rec.n > 0) s.samples = a->samples.ptr + step * a->rec.n;
-            check_cuda(dev::launch_speed_stage(a->N, a->fp32, s, stream), "speed stage launch");
+            check_cuda(launch_speed(a, s, stream), "speed stage launch");
             ++launches;
             in = 1 - in;
         }
@@ -299,6 +312,8 @@ ndg_status ndg_adjoint_create(ndg_ctx* ctx, int32_t n_receivers, const double* r
         check_cuda(dev::prepare_speed_kernels(a->N, false), "kernel attributes");
         check_cuda(dev::prepare_speed_kernels(a->N, true), "kernel attributes");
         check_cuda(dev::prepare_kernels_f32(a->N), "kernel attributes");
+        for (bool f32 : {false, true})
+            if (dev::line_kernel_runs(a->N, f32, a->K)) check_cuda(dev::prepare_speed_line(a->N, f32), "kernel attributes");
         check_cuda(cudaEventCreate(&a->ev[0]), "event");
         check_cuda(cudaEventCreate(&a->ev[1]), "event");
         check_cuda(cudaStreamSynchronize(s), "adjoint setup");
@@ -595,7 +610,9 @@ ndg_status ndg_adjoint_operator(ndg_adjoint* adj, const double* x, const double*
         dev::SpeedStageArgs f = speed_args(adj, 0, 0, 0.0);
         f.gdt = 0.0;
         f.G_out = adj->G.ptr;
-        check_cuda(dev::launch_speed_stage(adj->N, adj->fp32, f, s), "speed stage launch");
+        check_cuda(launch_speed(adj, f, s), "speed stage launch");
+        // the line kernel's k of a first stage is G
+        if (adj->line()) check_cuda(cudaMemcpyAsync(adj->G.ptr, adj->k.ptr, state * sizeof(double), cudaMemcpyDeviceToDevice, s), "operator result");
         // L^T y: publish the adjoint far traces of y (mu = 0, mu' = lq = y),
         // then one adjoint stage with mu = lk = y, lq = 0 and qs = x.
         zero_adjoint_traces(adj, 0);
@@ -650,7 +667,7 @@ ndg_status ndg_adjoint_time_stage(ndg_adjoint* adj, int32_t which, int32_t n_lau
             if (which < 2) {
                 dev::SpeedStageArgs a = speed_args(adj, 1, in, adj->dt);
                 if (which == 1) a.q_save = adj->seg.ptr;
-                check_cuda(dev::launch_speed_stage(adj->N, adj->fp32, a, s), "speed stage launch");
+                check_cuda(launch_speed(adj, a, s), "speed stage launch");
             } else {
                 dev::AdjointStageArgs a = adjoint_args(adj, in);
                 a.qs = adj->seg.ptr;

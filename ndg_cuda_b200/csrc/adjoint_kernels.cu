@@ -131,20 +131,6 @@ static AdjCoeffs<N, R> make_adj_coeffs() {
     return c;
 }
 
-// Pressure at the receivers of a tile, one warp: sum of w_r . p over the
-// element's nodes, lanes striding the nodes, then a shuffle reduction in a
-// fixed order (the same result wherever it is evaluated). FP64 in both forms.
-// Receiver sample sum_i w_i p_i over an element's nodes, with the element's
-// tile block p laid out in rows of pitch P (node i of n per row).
-template <int n, int P>
-__device__ __forceinline__ double receiver_value(const double* __restrict__ w, const double* p, int lane) {
-    double s = 0.0;
-    for (int i = lane; i < n * n; i += 32) s = fma(w[i], p[(i / n) * P + i % n], s);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    return s;
-}
-
 // ---------------------------------------------------------------------------
 // Forward stage with a wave speed per element, one thread per (field,
 // element, line), the line fastest: the FP64 q tile, then R arrays
@@ -221,6 +207,7 @@ __global__ void __launch_bounds__(SpeedTile<N, R>::kThreads) speed_stage_kernel(
     const bool active = f < 3 && e < ne;
     const int64_t ge = e0 + e;
 
+    pdl_wait();
     // q tile: warps take (field, element) blocks, lanes their nodes.
     const int warp = tid >> 5, lane = tid & 31;
     int lane_node[T::kLaneIters];
@@ -420,6 +407,7 @@ __global__ void __launch_bounds__(SpeedTile<N, R>::kThreads) speed_stage_kernel(
     }
     __syncthreads();
 
+    pdl_launch_dependents();
     if (active) {
         const double* row = qs + f * QSd + e * ESd + m * P;
         const double* cl = qs + f * QSd + e * ESd + m;
@@ -554,6 +542,7 @@ __global__ void __launch_bounds__(AdjTile<N, R>::kThreads) adjoint_stage_kernel(
     const bool active = f < 3 && e < ne;
     const int64_t ge = e0 + e;
 
+    pdl_wait();
     // Prologue: asynchronous copies of the lq and qs tiles (warps take
     // (field, element) blocks, lanes their nodes); adjoint far traces of the
     // neighbours, metrics, J, edge metrics and face speeds.
@@ -839,6 +828,7 @@ __global__ void __launch_bounds__(AdjTile<N, R>::kThreads) adjoint_stage_kernel(
     }
     __syncthreads();
 
+    pdl_launch_dependents();
     // Lift transpose of nu' on the four sides (column m: sides 1, 3; row m:
     // sides 2, 0); per element, the c-derivative accumulators (FP64).
     if (active) {
@@ -923,15 +913,15 @@ static cudaError_t prepare_speed_t() {
 template <int N, typename R>
 static cudaError_t launch_speed_stage_t(const SpeedStageArgs& a, cudaStream_t stream) {
     using T = SpeedTile<N, R>;
-    speed_stage_kernel<N, R><<<static_cast<unsigned>((a.n_elements + T::EPB - 1) / T::EPB), T::kThreads, T::kBytes, stream>>>(a, make_speed_coeffs<N, R>());
-    return cudaGetLastError();
+    return launch_dependent(speed_stage_kernel<N, R>, dim3(static_cast<unsigned>((a.n_elements + T::EPB - 1) / T::EPB)), T::kThreads, T::kBytes, stream, a,
+                            make_speed_coeffs<N, R>());
 }
 
 template <int N, typename R>
 static cudaError_t launch_adjoint_stage_t(const AdjointStageArgs& a, cudaStream_t stream) {
     using T = AdjTile<N, R>;
-    adjoint_stage_kernel<N, R><<<static_cast<unsigned>((a.n_elements + T::EPB - 1) / T::EPB), T::kThreads, T::kBytes, stream>>>(a, make_adj_coeffs<N, R>());
-    return cudaGetLastError();
+    return launch_dependent(adjoint_stage_kernel<N, R>, dim3(static_cast<unsigned>((a.n_elements + T::EPB - 1) / T::EPB)), T::kThreads, T::kBytes, stream, a,
+                            make_adj_coeffs<N, R>());
 }
 
 template <int N, typename R>

@@ -31,6 +31,20 @@ void set_last_error(const std::string& message) { g_last_error = message; }
 }  // namespace ndg
 
 namespace ndg {
+
+// Reads the kernels' error word (set when a bounded wait in a stage kernel
+// gave up); synchronises the stream.
+void check_device_error(ndg_ctx* c) {
+    if (!c->error.ptr) return;
+    unsigned err = 0;
+    check_cuda(cudaMemcpyAsync(&err, c->error.ptr, sizeof(err), cudaMemcpyDeviceToHost, c->stream), "error word readback");
+    check_cuda(cudaStreamSynchronize(c->stream), "error word readback");
+    if (err) {
+        check_cuda(cudaMemsetAsync(c->error.ptr, 0, sizeof(unsigned), c->stream), "memset");
+        fail(NDG_ERR_TIMEOUT, "a stage kernel gave up waiting for its tile copies; the state is not valid");
+    }
+}
+
 namespace {
 
 bool strict(const ndg_ctx* c) { return c->precision == NDG_FP64_STRICT; }
@@ -43,19 +57,6 @@ void drop_graphs(ndg_ctx* c) {
     for (auto& g : c->graph_many) {
         if (g) cudaGraphExecDestroy(g);
         g = nullptr;
-    }
-}
-
-// Reads the kernels' error word (set when a bounded wait in a stage kernel
-// gave up); synchronises the stream.
-void check_device_error(ndg_ctx* c) {
-    if (!c->error.ptr) return;
-    unsigned err = 0;
-    check_cuda(cudaMemcpyAsync(&err, c->error.ptr, sizeof(err), cudaMemcpyDeviceToHost, c->stream), "error word readback");
-    check_cuda(cudaStreamSynchronize(c->stream), "error word readback");
-    if (err) {
-        check_cuda(cudaMemsetAsync(c->error.ptr, 0, sizeof(unsigned), c->stream), "memset");
-        fail(NDG_ERR_TIMEOUT, "a stage kernel gave up waiting for its tile copies; the state is not valid");
     }
 }
 

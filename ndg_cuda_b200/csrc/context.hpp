@@ -183,6 +183,10 @@ struct ndg_ctx {
 
 namespace ndg {
 
+// Reads the kernels' error word (synchronises the stream) and fails when a
+// bounded wait gave up.
+void check_device_error(ndg_ctx* c);
+
 inline void require_device(const ndg_ctx* c) {
     if (c->device < 0) fail(NDG_ERR_INVALID_ARG, "this call needs a GPU context (device >= 0)");
 }

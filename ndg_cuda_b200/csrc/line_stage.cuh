@@ -38,6 +38,7 @@
 // (q and k) and registers.
 #pragma once
 
+#include "adjoint.cuh"
 #include "ndg_internal.hpp"
 #include "stage_common.cuh"
 #include "stage_kernels.cuh"
@@ -283,11 +284,15 @@ __device__ __forceinline__ void line_contract(const LineCoeffs<N, R>& cf, const 
     }
 }
 
-template <int N, typename R, int E>
-__global__ void __launch_bounds__(LineTile<N, R, E>::kThreads, LineTile<N, R, E>::kMinBlocks) line_stage_kernel(StageArgs a, const __grid_constant__ LineCoeffs<N, R> cf) {
+// Args: StageArgs, or SpeedStageArgs for the variable-speed stage of the
+// adjoint module (adjoint.cuh: the volume term times the element's speed, the
+// face flux times the face's, optional copies of the stage input and of the
+// receivers' pressure; one instance, no inflow sides).
+template <int N, typename R, int E, typename Args>
+__global__ void __launch_bounds__(LineTile<N, R, E>::kThreads, LineTile<N, R, E>::kMinBlocks) line_stage_kernel(Args a, const __grid_constant__ LineCoeffs<N, R> cf) {
     using T = LineTile<N, R, E>;
     constexpr int n = T::n, NN = T::NN, P = T::P, ES = T::ES, QS = T::QS, SE = T::SE;
-    constexpr bool F64 = std::is_same_v<R, double>;
+    constexpr bool F64 = std::is_same_v<R, double>, kSpeed = std::is_same_v<Args, SpeedStageArgs>;
     extern __shared__ __align__(128) double smem[];
     double* qs = smem + T::kQ;
     double* ks = smem + T::kK;
@@ -330,11 +335,17 @@ __global__ void __launch_bounds__(LineTile<N, R, E>::kThreads, LineTile<N, R, E>
     struct SidePlanEntry {
         int2 lk;
         double2 nv, c0, c1;
+        double speed;  // of the face (kSpeed)
     };
     const auto read_side = [&](int i) {
         const int64_t o = 4 * e0 + i;
-        return SidePlanEntry{a.link[o], a.normal[o], reinterpret_cast<const double2*>(a.corners)[o],
-                             reinterpret_cast<const double2*>(a.corners)[(o & ~int64_t{3}) + ((i + 1) & 3)]};
+        SidePlanEntry p{a.link[o], a.normal[o], reinterpret_cast<const double2*>(a.corners)[o],
+                        reinterpret_cast<const double2*>(a.corners)[(o & ~int64_t{3}) + ((i + 1) & 3)], 1.0};
+        if constexpr (kSpeed) {
+            p.speed = a.c[o >> 2];
+            if (((p.lk.y >> 2) & 7) == kInterior) p.speed = 0.5 * (p.speed + a.c[p.lk.x]);
+        }
+        return p;
     };
     const auto put_side = [&](int i, const SidePlanEntry& p) {
         const bool role = (p.lk.y >> 5) & 1;
@@ -344,6 +355,7 @@ __global__ void __launch_bounds__(LineTile<N, R, E>::kThreads, LineTile<N, R, E>
         side[o] = R(role ? -p.nv.x : p.nv.x);
         side[4 * E + o] = R(role ? -p.nv.y : p.nv.y);
         side[8 * E + o] = R(0.5) * sqrt(dx * dx + dy * dy);
+        if constexpr (kSpeed) side[8 * E + o] *= R(p.speed);
         side[12 * E + o] = dx;
         side[16 * E + o] = dy;
         to_s[o] = kind == kInterior ? (p.lk.x * 4 + (p.lk.y & 3)) : ~kind;
@@ -351,7 +363,8 @@ __global__ void __launch_bounds__(LineTile<N, R, E>::kThreads, LineTile<N, R, E>
     SidePlanEntry first_side{};
     if (tid < 4 * ne) first_side = read_side(tid);
     pdl_wait();
-    if (a.step_next && blockIdx.x == 0 && blockIdx.y == 0 && tid == 0) advance_step(a.step, a.step_next);
+    if constexpr (!kSpeed)
+        if (a.step_next && blockIdx.x == 0 && blockIdx.y == 0 && tid == 0) advance_step(a.step, a.step_next);
     if constexpr (T::kBulk) {
         if (tid == 0) {
             const uint32_t bytes = static_cast<uint32_t>(((ne + 1) & ~1) * NN * sizeof(double));
@@ -391,6 +404,30 @@ __global__ void __launch_bounds__(LineTile<N, R, E>::kThreads, LineTile<N, R, E>
     const R* xn = cf.xn;
     const R* lm = cf.lm;
     const R* lp = cf.lp;
+    R ce = 1;  // element speed
+    if constexpr (kSpeed) ce = active ? R(a.c[ge]) : R(1);
+    const auto scaled = [&](R v) {
+        if constexpr (kSpeed) return ce * v;
+        return v;
+    };
+    if constexpr (kSpeed) {
+        // The stage input, for the adjoint's gradient: out of the tile before
+        // the rows overwrite it.
+        if (a.q_save) {
+            if constexpr (T::kBulk) {
+                if (tid == 0) {
+                    const uint32_t bytes = static_cast<uint32_t>(((ne + 1) & ~1) * NN * sizeof(double));
+                    for (int f = 0; f < 3; ++f) bulk_store(a.q_save + (f * Kp + e0) * NN, qs + f * QS, bytes);
+                    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                }
+            } else {
+#pragma unroll
+                for (int f = 0; f < 3; ++f)
+#pragma unroll 4
+                    for (int i = tid; i < ne * NN; i += T::kThreads) a.q_save[(f * Kp + e0) * NN + i] = qs[f * QS + T::place(i)];
+            }
+        }
+    }
     const R* dxs = side + 12 * E + e;
     const R* dys = side + 16 * E + e;
 
@@ -418,14 +455,16 @@ __global__ void __launch_bounds__(LineTile<N, R, E>::kThreads, LineTile<N, R, E>
                     fu = nx * l0 - ny * l1;
                     fv = ny * l0 + nx * l1;
                 }
-            } else if (kind == kAnalytic) {
-                const double4 gq = a.inflow[4 * ge + s];
-                const double r = (static_cast<double>(xn[N - idx]) + 1.0) * 0.5;
-                double pd, ud, vd;
-                plane_wave(gq.z * r + gq.x * (1.0 - r), gq.w * r + gq.y * (1.0 - r), a.step[0] + a.rk_b * a.step[1], pd, ud, vd);
-                fp = R(pd);
-                fu = R(ud);
-                fv = R(vd);
+            } else if constexpr (!kSpeed) {
+                if (kind == kAnalytic) {
+                    const double4 gq = a.inflow[4 * ge + s];
+                    const double r = (static_cast<double>(xn[N - idx]) + 1.0) * 0.5;
+                    double pd, ud, vd;
+                    plane_wave(gq.z * r + gq.x * (1.0 - r), gq.w * r + gq.y * (1.0 - r), a.step[0] + a.rk_b * a.step[1], pd, ud, vd);
+                    fp = R(pd);
+                    fu = R(ud);
+                    fv = R(vd);
+                }
             }
             wR = characteristic(fp, fu, fv, -nx, -ny);
         }
@@ -474,13 +513,16 @@ __global__ void __launch_bounds__(LineTile<N, R, E>::kThreads, LineTile<N, R, E>
         };
 #pragma unroll
         for (int i = 0; i < n; ++i) {
-            const R xe = x_eta(xn[i]), ye = y_eta(xn[i]);
+            const R xe = scaled(x_eta(xn[i])), ye = scaled(y_eta(xn[i]));
             const R p = x[0][i];
             x[0][i] = ye * x[1][i] - xe * x[2][i];
             x[1][i] = ye * p;
             x[2][i] = -xe * p;
         }
         line_contract<N, R>(cf, x, Fr, Fl, upd);
+    }
+    if constexpr (kSpeed && T::kBulk) {
+        if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
     }
     __syncthreads();
     if (active) {
@@ -489,7 +531,11 @@ __global__ void __launch_bounds__(LineTile<N, R, E>::kThreads, LineTile<N, R, E>
         // characteristics of the new q.
         double* Q = qs + e * ES + m * P;
         double* Kr = ks + e * ES + m * P;
-        const double gdt = a.rk_g * a.step[1];
+        double gdt;
+        if constexpr (kSpeed)
+            gdt = a.gdt;
+        else
+            gdt = a.rk_g * a.step[1];
         R x[3][n];
         R tt[3] = {0, 0, 0}, tb[3] = {0, 0, 0};
 #pragma unroll
@@ -521,7 +567,7 @@ __global__ void __launch_bounds__(LineTile<N, R, E>::kThreads, LineTile<N, R, E>
         };
 #pragma unroll
         for (int j = 0; j < n; ++j) {
-            const R xx = x_xi(xn[j]), yx = y_xi(xn[j]);
+            const R xx = scaled(x_xi(xn[j])), yx = scaled(y_xi(xn[j]));
             const R p = x[0][j];
             x[0][j] = xx * x[2][j] - yx * x[1][j];
             x[1][j] = -yx * p;
@@ -570,6 +616,17 @@ __global__ void __launch_bounds__(LineTile<N, R, E>::kThreads, LineTile<N, R, E>
             }
         send(1, m, tr[0], tr[1], tr[2]);
         send(3, N - m, tl[0], tl[1], tl[2]);
+    }
+    if constexpr (kSpeed) {
+        // Receivers' pressure of the new q, one warp, in a fixed order.
+        if (a.samples && tid < 32) {
+            for (int r = 0; r < a.rec.n; ++r) {
+                const int64_t el = a.rec.elem[r] - e0;
+                if (el < 0 || el >= ne) continue;
+                const double v = receiver_value<n, P>(a.rec.w + static_cast<int64_t>(r) * NN, qs + el * ES, tid);
+                if (tid == 0) a.samples[r] = v;
+            }
+        }
     }
     if constexpr (T::kBulk) {
         if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");

@@ -21,7 +21,7 @@ constexpr bool usable() {
 template <int N, int E>
 cudaError_t prepare() {
     if constexpr (usable<N, E>())
-        return cudaFuncSetAttribute(line_stage_kernel<N, R, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(LineTile<N, R, E>::kBytes));
+        return cudaFuncSetAttribute(line_stage_kernel<N, R, E, StageArgs>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(LineTile<N, R, E>::kBytes));
     else
         return cudaErrorInvalidValue;
 }
@@ -31,7 +31,7 @@ cudaError_t launch(const StageArgs& a, cudaStream_t stream) {
     if constexpr (usable<N, E>()) {
         using T = LineTile<N, R, E>;
         const dim3 grid(static_cast<unsigned>((a.n_elements + E - 1) / E), static_cast<unsigned>(a.n_instances));
-        return launch_dependent(line_stage_kernel<N, R, E>, grid, T::kThreads, T::kBytes, stream, a, make_line_coeffs<N, R>());
+        return launch_dependent(line_stage_kernel<N, R, E, StageArgs>, grid, T::kThreads, T::kBytes, stream, a, make_line_coeffs<N, R>());
     } else {
         return cudaErrorInvalidValue;
     }

@@ -95,3 +95,35 @@ def test_line_kernel_against_the_oracle(N):
     for f in ("p", "u", "v"):
         assert rel_l2(m.get_field(f), o.field(f)) < 1e-12, f
     m.close()
+
+
+@pytest.mark.parametrize("precision", [ndg.FP64, ndg.FP32])
+@pytest.mark.parametrize("N", [4, 5, 7, 8, 10, 11])
+@pytest.mark.parametrize("boundary", ["wall", "periodic"])
+def test_variable_speed_line_stage(N, precision, boundary):
+    """The variable-speed stage in the line kernel: the operator and the
+    gradient (kept stage inputs, samples, recomputation) against the oracle's
+    CPU adjoint, to the tolerances of the adjoint's own tests."""
+    from tests import adjoint_setup as A
+    kw = dict(boundary=meshgen.WALL) if boundary == "wall" else dict(x_periodic=True, y_periodic=True)
+    zone = meshgen.uniform_zone(41, order="rowmajor", jitter=0.1, seed=2, **kw)
+    rng = np.random.default_rng(N)
+    c = 1.0 + 0.2 * rng.random(41 * 41)
+    xy = A.circle_receivers(5, 0.6)
+    mesh = ndg.Mesh2D_t(zone, N)
+    adj = ndg.Adjoint2D_t(mesh, xy, speed=c, precision=precision)
+    o, el, w = A.oracle_problem(zone, N, c, xy)
+    x, y = rng.standard_normal(3 * mesh.field_size), rng.standard_normal(3 * mesh.field_size)
+    Lx, LTy, dc = adj.operator(x, y)
+    assert rel_l2(Lx, o.operator(x)) < (1e-12 if precision == ndg.FP64 else 1e-6)
+    p0 = A.gaussian_pulse(zone, N, sigma=0.3)
+    dt, steps = adj.delta_t(0.5), 5
+    target = 0.1 * rng.standard_normal((steps + 1, el.size))
+    J, samples = adj.forward(p0, dt, steps, targets=target, checkpoint_interval=2)
+    g = adj.backward()
+    ref = o.adjoint_solve(p0, dt, steps, el, w, targets=target)
+    assert rel_l2(samples, ref["samples"]) < (1e-12 if precision == ndg.FP64 else 1e-6)
+    for k in ("p0", "u0", "v0", "c"):
+        assert rel_l2(g[k], ref[k]) < (1e-10 if precision == ndg.FP64 else 1e-4), k
+    adj.close()
+    mesh.close()
