@@ -36,8 +36,8 @@ struct ndg_adjoint {
     cudaEvent_t evr[2] = {nullptr, nullptr}, eva[2] = {nullptr, nullptr}, evs = nullptr;
     ndg::DeviceBuffer<float> tr_f[2], atr_f[2];  // traces of the FP32 form
     bool fp32 = false;
-    // The forward stage runs the line kernel in this form (by the rule of the
-    // uniform stage), with its characteristics in tr / tr_f.
+    // The forward and adjoint stages run the line kernels in this form (by the
+    // rule of the uniform stage), with one value per side node in tr and atr.
     bool line() const { return ctx->seams_opposite && ndg::dev::line_kernel_runs(N, fp32, K); }
     ndg::dev::Receivers rec{};
     // the last forward
@@ -162,8 +162,13 @@ dev::AdjointStageArgs adjoint_args(ndg_adjoint* a, int in) {
     s.c = a->c.ptr;
     s.n_elements = a->K;
     s.field_stride = a->Kp;
+    s.error = c->error.ptr;
     s.rec = a->rec;
     return s;
+}
+
+cudaError_t launch_adjoint(ndg_adjoint* a, const dev::AdjointStageArgs& s, cudaStream_t stream) {
+    return a->line() ? dev::launch_adjoint_line(a->N, a->fp32, s, stream) : dev::launch_adjoint_stage(a->N, a->fp32, s, stream);
 }
 
 void launch_traces_of_q(ndg_adjoint* a, int out, cudaStream_t stream = nullptr) {
@@ -313,7 +318,10 @@ ndg_status ndg_adjoint_create(ndg_ctx* ctx, int32_t n_receivers, const double* r
         check_cuda(dev::prepare_speed_kernels(a->N, true), "kernel attributes");
         check_cuda(dev::prepare_kernels_f32(a->N), "kernel attributes");
         for (bool f32 : {false, true})
-            if (dev::line_kernel_runs(a->N, f32, a->K)) check_cuda(dev::prepare_speed_line(a->N, f32), "kernel attributes");
+            if (dev::line_kernel_runs(a->N, f32, a->K)) {
+                check_cuda(dev::prepare_speed_line(a->N, f32), "kernel attributes");
+                check_cuda(dev::prepare_adjoint_line(a->N, f32), "kernel attributes");
+            }
         check_cuda(cudaEventCreate(&a->ev[0]), "event");
         check_cuda(cudaEventCreate(&a->ev[1]), "event");
         check_cuda(cudaStreamSynchronize(s), "adjoint setup");
@@ -548,7 +556,7 @@ ndg_status ndg_adjoint_backward(ndg_adjoint* adj, double* grad_p0, double* grad_
                 a.inject = R > 0;
                 a.target = adj->targets.ptr + n * R;
                 a.wdt = adj->dt;
-                check_cuda(dev::launch_adjoint_stage(adj->N, adj->fp32, a, as), "adjoint stage launch");
+                check_cuda(launch_adjoint(adj, a, as), "adjoint stage launch");
                 ++launches;
                 ain = 1 - ain;
             }
@@ -562,7 +570,7 @@ ndg_status ndg_adjoint_backward(ndg_adjoint* adj, double* grad_p0, double* grad_
                     a.inject = (m == 0 && step - 1 >= 1 && R > 0) ? 1 : 0;
                     a.target = adj->targets.ptr + (step - 1) * R;
                     a.wdt = adj->dt;
-                    check_cuda(dev::launch_adjoint_stage(adj->N, adj->fp32, a, as), "adjoint stage launch");
+                    check_cuda(launch_adjoint(adj, a, as), "adjoint stage launch");
                     ++launches;
                     ain = 1 - ain;
                 }
@@ -622,13 +630,13 @@ ndg_status ndg_adjoint_operator(ndg_adjoint* adj, const double* x, const double*
         dev::AdjointStageArgs a = adjoint_args(adj, 0);
         a.qs = adj->q.ptr;
         a.gdt_next = 1.0;
-        check_cuda(dev::launch_adjoint_stage(adj->N, adj->fp32, a, s), "adjoint stage launch");
+        check_cuda(launch_adjoint(adj, a, s), "adjoint stage launch");
         check_cuda(cudaMemsetAsync(adj->acc.ptr, 0, adj->acc.count * sizeof(double), s), "memset");
         upload_state(adj, adj->lq.ptr, none);
         upload_state(adj, adj->lk.ptr, yf);
         a = adjoint_args(adj, 1);
         a.qs = adj->q.ptr;
-        check_cuda(dev::launch_adjoint_stage(adj->N, adj->fp32, a, s), "adjoint stage launch");
+        check_cuda(launch_adjoint(adj, a, s), "adjoint stage launch");
         check_cuda(dev::launch_speed_gradient(adj->acc.ptr, reinterpret_cast<const int2*>(c->link.ptr), adj->K, adj->grad.ptr, s), "gradient kernel");
         check_kernel_error(adj);
         for (int ff = 0; ff < 3; ++ff) {
@@ -674,7 +682,7 @@ ndg_status ndg_adjoint_time_stage(ndg_adjoint* adj, int32_t which, int32_t n_lau
                 a.rk_a = kRkA[1];
                 a.gdt = kRkG[1] * adj->dt;
                 a.gdt_next = kRkG[0] * adj->dt;
-                check_cuda(dev::launch_adjoint_stage(adj->N, adj->fp32, a, s), "adjoint stage launch");
+                check_cuda(launch_adjoint(adj, a, s), "adjoint stage launch");
             }
             check_cuda(cudaEventRecord(ev[static_cast<size_t>(2 * i + 1)], s), "cudaEventRecord");
             in = 1 - in;

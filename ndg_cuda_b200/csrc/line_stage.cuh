@@ -284,6 +284,60 @@ __device__ __forceinline__ void line_contract(const LineCoeffs<N, R>& cf, const 
     }
 }
 
+// The same product without a lift.
+template <int N, typename R, typename Out>
+__device__ __forceinline__ void line_product(const LineCoeffs<N, R>& cf, const R (&x)[3][N + 1], Out&& out) {
+    constexpr int n = N + 1, H = n / 2, HO = n - H;
+    if constexpr (LineCoeffs<N, R>::kEvenOdd) {
+        constexpr int C = HO < 5 ? HO : 5;
+        R e[3][HO], o[3][H];
+#pragma unroll
+        for (int f = 0; f < 3; ++f) {
+#pragma unroll
+            for (int j = 0; j < H; ++j) {
+                e[f][j] = x[f][j] + x[f][n - 1 - j];
+                o[f][j] = x[f][j] - x[f][n - 1 - j];
+            }
+            if constexpr (HO > H) e[f][H] = x[f][H];
+        }
+#pragma unroll
+        for (int i0 = 0; i0 < HO; i0 += C) {
+            R A[3][C], S[3][C];
+#pragma unroll
+            for (int j = 0; j < HO; ++j)
+#pragma unroll
+                for (int c = 0; c < C; ++c)
+#pragma unroll
+                    for (int f = 0; f < 3; ++f) {
+                        if (i0 + c < H) A[f][c] = j == 0 ? cf.ea[(i0 + c) * HO] * e[f][0] : fma(cf.ea[(i0 + c) * HO + j], e[f][j], A[f][c]);
+                        if (i0 + c < HO && j < H) S[f][c] = j == 0 ? cf.so[(i0 + c) * H] * o[f][0] : fma(cf.so[(i0 + c) * H + j], o[f][j], S[f][c]);
+                    }
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                const int i = i0 + c;
+#pragma unroll
+                for (int f = 0; f < 3; ++f)
+                    if (i < HO) out(f, i, i < H ? S[f][c] + A[f][c] : S[f][c]);
+#pragma unroll
+                for (int f = 0; f < 3; ++f)
+                    if (i < H) out(f, n - 1 - i, S[f][c] - A[f][c]);
+            }
+        }
+    } else {
+        R A[3][n];
+#pragma unroll
+        for (int j = 0; j < n; ++j)
+#pragma unroll
+            for (int i = 0; i < n; ++i)
+#pragma unroll
+                for (int f = 0; f < 3; ++f) A[f][i] = j == 0 ? cf.dhat[i * n] * x[f][0] : fma(cf.dhat[i * n + j], x[f][j], A[f][i]);
+#pragma unroll
+        for (int i = 0; i < n; ++i)
+#pragma unroll
+            for (int f = 0; f < 3; ++f) out(f, i, A[f][i]);
+    }
+}
+
 // Args: StageArgs, or SpeedStageArgs for the variable-speed stage of the
 // adjoint module (adjoint.cuh: the volume term times the element's speed, the
 // face flux times the face's, optional copies of the stage input and of the
