@@ -15,9 +15,9 @@
 // b: a third of the trace traffic of three components, as in the forward.
 //
 // Measured, backward of 60 steps with checkpoints every 20 at 96 x 96 (its
-// recomputation included), ms, against three threads a line: FP64 N = 4 2.45
-// (4.65), N = 6 4.29 (6.86), N = 7 5.46 (7.76), N = 8 7.31 (10.39), N = 9 10.03
-// (13.68); FP32 form N = 4 2.63 (3.41), N = 6 4.68 (6.23), N = 8 7.50 (9.10).
+// recomputation included), ms, against three threads a line: FP64 N = 4 2.00
+// (4.65), N = 6 3.52 (6.86), N = 7 5.07 (7.76), N = 8 5.89 (10.39), N = 9 10.03
+// (13.68); FP32 form N = 4 2.15 (3.41), N = 6 3.98 (6.23), N = 8 6.21 (9.10).
 // Nine field tiles an element bound the tiles per SM; latency is what is left.
 #include "adjoint.cuh"
 #include "line_stage.cuh"
@@ -383,11 +383,13 @@ __global__ void __launch_bounds__(AdjLineTile<N, R, E>::kThreads, AdjLineTile<N,
     }
 }
 
-// Elements a tile: 8 up to order 10 (4: N = 8 8.78 ms in the measure above),
-// 4 above, where 8 leave one tile an SM.
+// Elements a tile, by the measure above (96 x 96, ms, with 16 / 8 / 4): FP64 N =
+// 4 2.00 / 2.45 / 2.61, N = 6 3.52 / 4.29 / 4.24, N = 7 5.07 / 5.46 / 5.53, N =
+// 8 5.89 / 7.31 / 8.78, N = 9 10.71 / 10.03 / 10.19; above order 10 a tile of 8
+// is alone on its SM.
 template <int N>
 constexpr int elements() {
-    return N <= 10 ? 8 : 4;
+    return N <= 8 || N == 10 ? 16 : (N <= 10 ? 8 : 4);
 }
 
 template <int N, typename R>
