@@ -194,7 +194,11 @@ ndg_status ndg_mesh_field_size(const ndg_ctx* ctx, int64_t* n_values);
  * plane wave g(x, 0) in every instance; G and the RK register are zeroed. */
 ndg_status ndg_initial_conditions(ndg_ctx* ctx);
 /* Copies one field of one instance from/to host memory (field_size values).
- * instance < 0 addresses all instances back to back. */
+ * instance < 0 addresses all instances back to back. ndg_set_field's copy is
+ * on the context's stream: a pinned buffer may be reused once a stepping call
+ * (ndg_stage, ndg_run, ndg_solve, ndg_pre_condition) or ndg_ctx_synchronize
+ * has returned; they wait for the stream's work before them. Stepping calls
+ * cannot be captured into a graph (NDG_ERR_CUDA on a capturing stream). */
 ndg_status ndg_set_field(ndg_ctx* ctx, int32_t instance, int32_t field, const double* values);
 ndg_status ndg_get_field(ndg_ctx* ctx, int32_t instance, int32_t field, double* values);
 

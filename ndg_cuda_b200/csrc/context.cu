@@ -319,6 +319,29 @@ void set_step(ndg_ctx* c, double time, double dt, double t_end) {
     ++c->launches;
 }
 
+// A stepping call's work: the step state, then `enqueue`'s launches. It returns
+// when everything that was on the stream before it is complete (not its own
+// launches), so a caller may reuse a pinned buffer it gave to ndg_set_field;
+// waiting after the launches costs the device no gap. Refused on a capturing
+// stream: the captured launches could not be replayed with the host's parity,
+// time and graphs.
+template <typename Enqueue>
+void step_work(ndg_ctx* c, double time, double dt, double t_end, Enqueue&& enqueue) {
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    check_cuda(cudaStreamIsCapturing(c->stream, &capturing), "stream capture status");
+    if (capturing != cudaStreamCaptureStatusNone) fail(NDG_ERR_CUDA, "stepping calls cannot be captured");
+    if (!c->before_step) check_cuda(cudaEventCreateWithFlags(&c->before_step, cudaEventDisableTiming), "cudaEventCreate");
+    check_cuda(cudaEventRecord(c->before_step, c->stream), "cudaEventRecord");
+    try {
+        set_step(c, time, dt, t_end);
+        enqueue();
+    } catch (...) {
+        cudaEventSynchronize(c->before_step);
+        throw;
+    }
+    check_cuda(cudaEventSynchronize(c->before_step), "work before the step");
+}
+
 // Steps captured as CUDA graphs: three stages each, and on mixed-order meshes
 // the time update (the uniform kernels' last stage does it). A step flips the
 // trace buffer an odd number of times, so there are two graphs by parity. The
@@ -1348,9 +1371,10 @@ ndg_status ndg_stage(ndg_ctx* ctx, int32_t m, double time, double dt) {
         require_device(ctx);
         if (m < 0 || m > 2) fail(NDG_ERR_INVALID_ARG, "stage index must be 0, 1 or 2");
         make_current(ctx);
-        set_step(ctx, time, dt, std::numeric_limits<double>::infinity());
-        ensure_traces(ctx);
-        launch_stage(ctx, m);
+        step_work(ctx, time, dt, std::numeric_limits<double>::infinity(), [&] {
+            ensure_traces(ctx);
+            launch_stage(ctx, m);
+        });
     });
 }
 
@@ -1361,8 +1385,7 @@ ndg_status ndg_run(ndg_ctx* ctx, int64_t n_steps, double* time) {
         if (n_steps < 0) fail(NDG_ERR_INVALID_ARG, "n_steps must be >= 0");
         make_current(ctx);
         const double t0 = time ? *time : 0.0;
-        set_step(ctx, t0, ctx->dt_mesh, std::numeric_limits<double>::infinity());
-        run_steps(ctx, n_steps);
+        step_work(ctx, t0, ctx->dt_mesh, std::numeric_limits<double>::infinity(), [&] { run_steps(ctx, n_steps); });
         // The device advances time by the same FP64 additions.
         double t = t0;
         for (int64_t s = 0; s < n_steps; ++s) t += ctx->dt_mesh;
@@ -1394,8 +1417,7 @@ ndg_status ndg_solve(ndg_ctx* ctx, double t_end, double* time, int64_t* n_steps)
                 ++n;
             }
             const double dt0 = (c0 + ctx->dt_mesh > t_end) ? t_end - c0 : ctx->dt_mesh;
-            set_step(ctx, c0, dt0, t_end);
-            run_steps(ctx, n);
+            step_work(ctx, c0, dt0, t_end, [&] { run_steps(ctx, n); });
             steps += n;
             if (interval > 0 && n == limit) {
                 estimate(ctx);
@@ -1422,8 +1444,7 @@ ndg_status ndg_pre_condition(ndg_ctx* ctx, int64_t n_adaptivity_steps, int64_t p
         double t = 0.0;
         int64_t steps = 0;
         for (int64_t a = 0; a < n_adaptivity_steps; ++a) {
-            set_step(ctx, t, ctx->dt_mesh, std::numeric_limits<double>::infinity());
-            run_steps(ctx, pre_condition_interval);
+            step_work(ctx, t, ctx->dt_mesh, std::numeric_limits<double>::infinity(), [&] { run_steps(ctx, pre_condition_interval); });
             for (int64_t s = 0; s < pre_condition_interval; ++s) t += ctx->dt_mesh;
             steps += pre_condition_interval;
             estimate(ctx);

@@ -162,6 +162,7 @@ struct ndg_ctx {
     // Graphs by trace-buffer parity: one step, and kGraphSteps steps.
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
     cudaGraphExec_t graph_many[2] = {nullptr, nullptr};
+    cudaEvent_t before_step = nullptr;  // end of the stream's work before the current stepping call
     int64_t launches = 0;
     // Incremented whenever the topology or its device plan changes (load,
     // adaptation): objects built on the mesh (adjoint problems) check it.
@@ -175,6 +176,7 @@ struct ndg_ctx {
             if (g) cudaGraphExecDestroy(g);
         for (auto& g : graph_many)
             if (g) cudaGraphExecDestroy(g);
+        if (before_step) cudaEventDestroy(before_step);
         for (auto& e : aux_events) cudaEventDestroy(e);
         for (auto& st : aux_streams) cudaStreamDestroy(st);
         if (own_stream && stream) cudaStreamDestroy(stream);
