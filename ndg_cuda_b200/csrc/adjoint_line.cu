@@ -60,9 +60,9 @@ struct AdjLineTile {
     using L = LineTile<N, R, E>;
     static constexpr int n = N + 1, QS = L::QS;
     static constexpr int kThreads = L::kThreads;
-    static constexpr int kDoubles = 9 * QS + (9 * QS) % 2 + kMaxReceivers + (E + 1) / 2 * 2;  // lq, lk (mu), qs (nu'); residuals; receiver masks
-    static constexpr int kRes = 9 * QS + (9 * QS) % 2, kMask = kRes + kMaxReceivers;
-    static constexpr int kFar = 0, kSide = (E * L::SE + 1) / 2 * 2, kSum = kSide + 7 * 4 * E, kRs = (kSum + 5 * n * E + 3) / 4 * 4;
+    static constexpr int kRes = 9 * QS + (9 * QS) % 2, kMask = kRes + kMaxReceivers, kVol = kMask + (E + 1) / 2 * 2;
+    static constexpr int kDoubles = kVol + (n * E + 1) / 2 * 2;  // lq, lk (mu), qs (nu'); residuals; receiver masks; volume sums
+    static constexpr int kFar = 0, kSide = (E * L::SE + 1) / 2 * 2, kSum = kSide + 7 * 4 * E, kRs = (kSum + 4 * n * E + 3) / 4 * 4;
     static constexpr size_t kBytes = sizeof(double) * kDoubles + 16 + sizeof(R) * kRs + sizeof(int) * 4 * E;
     static constexpr int kFit = static_cast<int>((232448 - (L::kBulk ? 0 : 24 * 1024)) / (kBytes + 1024));
     static constexpr int kByRegs = 65536 / (kThreads * 128);
@@ -87,7 +87,8 @@ __global__ void __launch_bounds__(AdjLineTile<N, R, E>::kThreads, AdjLineTile<N,
     R* rs = reinterpret_cast<R*>(bar + 2);
     R* far_s = rs + A::kFar;
     R* side = rs + A::kSide;  // [nx, ny, edge metric, face speed, dx, dy, ghost scale][side][element]
-    R* sum_s = rs + A::kSum;  // [volume, side 0..3][line][element] of the speed derivative
+    R* sum_s = rs + A::kSum;         // [side][line][element] of the speed derivative
+    double* vol_s = smem + A::kVol;  // [line][element], its volume part
     int* to_s = reinterpret_cast<int*>(rs + A::kRs);
     const int tid = threadIdx.x;
     const int64_t K = a.n_elements, Kp = a.field_stride;
@@ -228,7 +229,16 @@ __global__ void __launch_bounds__(AdjLineTile<N, R, E>::kThreads, AdjLineTile<N,
         halves(s, l, hp, hn);
         atr_out[static_cast<int64_t>(to) * n + (N - idx)] = hn - hp;
     };
-    R vdot = 0;
+    // Volume part of the speed derivative on this thread's column and row: in
+    // the FP32 form one FP32 sum per field, joined in FP64. One sum over the
+    // three fields is further from FP64 (N = 8, 40 x 40: 2.48e-7 relative RMS
+    // against 2.03e-7; three threads a line 1.95e-7); backward of 60 steps at
+    // 96 x 96 6.11 -> 6.14 ms (N = 5 2.97 -> 3.03).
+    R vdot[F64 ? 1 : 3] = {};
+    const auto volume = [&](int f, R q, R d) {
+        R& v = vdot[F64 ? 0 : f];
+        v = fma(q, d, v);
+    };
 
     if (active) {
         double* Lc = ls + e * ES + m;
@@ -255,8 +265,8 @@ __global__ void __launch_bounds__(AdjLineTile<N, R, E>::kThreads, AdjLineTile<N,
             }
         }
         R t1[3], t3[3];
-        sum_s[(2 * n + m) * E + e] = side_adjoint(1, m, l1, r, t1);
-        sum_s[(4 * n + (N - m)) * E + e] = side_adjoint(3, N - m, l3, l, t3);
+        sum_s[(1 * n + m) * E + e] = side_adjoint(1, m, l1, r, t1);
+        sum_s[(3 * n + (N - m)) * E + e] = side_adjoint(3, N - m, l3, l, t3);
         R y[3];
         line_product<N, R>(cf.t, x, [&](int f, int i, R v) {
             y[f] = v;
@@ -264,7 +274,9 @@ __global__ void __launch_bounds__(AdjLineTile<N, R, E>::kThreads, AdjLineTile<N,
             const R xe = x_eta(xn[i]), ye = y_eta(xn[i]);
             const R dp = ye * y[1] - xe * y[2], du = ye * y[0], dv = -xe * y[0];
             const int o = i * P;
-            vdot = fma(R(Q[o]), dp, fma(R(Q[QS + o]), du, fma(R(Q[2 * QS + o]), dv, vdot)));
+            volume(2, R(Q[2 * QS + o]), dv);
+            volume(1, R(Q[QS + o]), du);
+            volume(0, R(Q[o]), dp);
             Lc[o] += static_cast<double>(ce * dp) + static_cast<double>(fma(lp[i], t1[0], lm[i] * t3[0]));
             Lc[QS + o] += static_cast<double>(ce * du) + static_cast<double>(fma(lp[i], t1[1], lm[i] * t3[1]));
             Lc[2 * QS + o] += static_cast<double>(ce * dv) + static_cast<double>(fma(lp[i], t1[2], lm[i] * t3[2]));
@@ -293,8 +305,8 @@ __global__ void __launch_bounds__(AdjLineTile<N, R, E>::kThreads, AdjLineTile<N,
             }
         }
         R t2[3], t0[3];
-        sum_s[(3 * n + (N - m)) * E + e] = side_adjoint(2, N - m, l2, tp, t2);
-        sum_s[(1 * n + m) * E + e] = side_adjoint(0, m, l0, bt, t0);
+        sum_s[(2 * n + (N - m)) * E + e] = side_adjoint(2, N - m, l2, tp, t2);
+        sum_s[m * E + e] = side_adjoint(0, m, l0, bt, t0);
 #pragma unroll
         for (int f = 0; f < 3; ++f) l2[f] = l0[f] = 0;
         const unsigned long long mask0 = rmask[e];
@@ -308,7 +320,7 @@ __global__ void __launch_bounds__(AdjLineTile<N, R, E>::kThreads, AdjLineTile<N,
 #pragma unroll
             for (int g = 0; g < 3; ++g) {
                 const int o = g * QS + j;
-                vdot = fma(R(Q[o]), d[g], vdot);
+                volume(g, R(Q[o]), d[g]);
                 double lq = Lr[o] + (static_cast<double>(ce * d[g]) + static_cast<double>(fma(lp[j], t2[g], lm[j] * t0[g])));
                 if (g == 0) {
                     unsigned long long mask = mask0;
@@ -327,7 +339,10 @@ __global__ void __launch_bounds__(AdjLineTile<N, R, E>::kThreads, AdjLineTile<N,
                 l0[g] = fma(nu, cf.lmw[j], l0[g]);
             }
         });
-        sum_s[m * E + e] = vdot;
+        if constexpr (F64)
+            vol_s[m * E + e] = vdot[0];
+        else
+            vol_s[m * E + e] = (static_cast<double>(vdot[0]) + static_cast<double>(vdot[1])) + static_cast<double>(vdot[2]);
         publish(2, N - m, l2);
         publish(0, m, l0);
     }
@@ -374,7 +389,7 @@ __global__ void __launch_bounds__(AdjLineTile<N, R, E>::kThreads, AdjLineTile<N,
         const int w = i / E, el = i % E;
         if (el < ne) {
             double s = 0.0;
-            for (int j = 0; j < n; ++j) s += static_cast<double>(sum_s[(w * n + j) * E + el]);
+            for (int j = 0; j < n; ++j) s += w == 0 ? vol_s[j * E + el] : static_cast<double>(sum_s[((w - 1) * n + j) * E + el]);
             a.acc[(e0 + el) * 5 + w] += s;
         }
     }
