@@ -250,6 +250,7 @@ void require_form(ndg_ctx* c) {
     }
 }
 
+// A stage outside a step: the step state is in both buffers (set_step, hold_step).
 void launch_stage(ndg_ctx* c, int m) {
     require_form(c);
     check_cuda(issue_stage(c, m, c->cur, c->general ? 0 : c->cur, false), "stage kernel launch");
@@ -313,10 +314,19 @@ void ensure_traces(ndg_ctx* c) {
     c->traces_valid = true;
 }
 
-// The step state of the next launch (of the buffer the current parity reads).
+// The step state, in both step buffers. Steps of the uniform path then advance
+// it from the buffer of the trace parity into the other one, so after them only
+// the buffer of `cur` is current.
 void set_step(ndg_ctx* c, double time, double dt, double t_end) {
-    check_cuda(dev::launch_set_step(c->step.ptr + (c->general ? 0 : 4 * c->cur), time, dt, c->dt_mesh, t_end, c->stream), "step state");
+    check_cuda(dev::launch_set_step(c->step.ptr, time, dt, c->dt_mesh, t_end, c->stream), "step state");
     ++c->launches;
+}
+
+// Brings the other step buffer up to date: before stages that do not advance
+// the state, which read the two buffers in turn, and before `cur` is reset.
+void hold_step(ndg_ctx* c) {
+    if (c->general || !c->step.ptr) return;
+    check_cuda(cudaMemcpyAsync(c->step.ptr + 4 * (1 - c->cur), c->step.ptr + 4 * c->cur, 4 * sizeof(double), cudaMemcpyDeviceToDevice, c->stream), "step state");
 }
 
 // A stepping call's work: the step state, then `enqueue`'s launches. It returns
@@ -441,6 +451,7 @@ Layout layout_of(const Topology& t) {
 // plan of the uniform path or the arrays of the general path.
 void upload_plan(ndg_ctx* c, const Layout& l) {
     const size_t inst = static_cast<size_t>(c->n_instances);
+    hold_step(c);
     c->general = l.general;
     c->block = l.block;
     c->field_size = l.field_size;
@@ -1466,6 +1477,7 @@ ndg_status ndg_time_stage(ndg_ctx* ctx, int32_t m, int32_t n_launches, double* a
         if (m < 0 || m > 2 || n_launches < 1 || !avg_ms) fail(NDG_ERR_INVALID_ARG, "bad stage timing request");
         make_current(ctx);
         ensure_traces(ctx);
+        hold_step(ctx);
         std::vector<cudaEvent_t> ev(static_cast<size_t>(2 * n_launches));
         for (auto& e : ev) check_cuda(cudaEventCreate(&e), "cudaEventCreate");
         for (int i = 0; i < n_launches; ++i) {
@@ -1533,6 +1545,7 @@ ndg_status ndg_autotune(ndg_ctx* ctx, int32_t n_launches, int32_t* elements_per_
         check_cuda(cudaMemcpyAsync(k0.ptr, ctx->k.ptr, values * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream), "state copy");
         std::vector<int> cand = tile_candidates(ctx);
         cand.insert(cand.begin(), 0);  // the default tile
+        hold_step(ctx);
         cudaEvent_t e0, e1;
         check_cuda(cudaEventCreate(&e0), "cudaEventCreate");
         check_cuda(cudaEventCreate(&e1), "cudaEventCreate");

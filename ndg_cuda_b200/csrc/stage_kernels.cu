@@ -195,7 +195,9 @@ __global__ void delta_t_kernel(const double* delta_xy_min, const int* elem_N, in
 // kernels do it themselves).
 __global__ void end_step_kernel(double* step) { advance_step(step, step); }
 
+// Both buffers of the step state, by threads 0 and 1.
 __global__ void set_step_kernel(double* step, double time, double dt, double dt_mesh, double t_end) {
+    step += 4 * threadIdx.x;
     step[0] = time;
     step[1] = dt;
     step[2] = dt_mesh;
@@ -450,7 +452,7 @@ cudaError_t launch_end_step(double* step, cudaStream_t stream) {
 }
 
 cudaError_t launch_set_step(double* step, double time, double dt, double dt_mesh, double t_end, cudaStream_t stream) {
-    set_step_kernel<<<1, 1, 0, stream>>>(step, time, dt, dt_mesh, t_end);
+    set_step_kernel<<<1, 2, 0, stream>>>(step, time, dt, dt_mesh, t_end);
     return cudaGetLastError();
 }
 

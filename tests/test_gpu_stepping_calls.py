@@ -79,3 +79,44 @@ def test_a_stepping_call_on_a_capturing_stream_is_refused():
     assert torch.equal(x, torch.ones_like(x))
     assert np.array_equal(_get(m), before)
     m.close()
+
+
+@pytest.mark.parametrize("N", [3, 6])
+@pytest.mark.parametrize("steps", [0, 1, 2, 9])
+def test_timed_stages_run_at_the_state_the_last_call_left(N, steps):
+    """ndg_time_stage's launches are stages at the time and step the last
+    stepping call left (the inflow boundary takes its values from them), in a
+    row, after autotuning and after the mesh became a mixed-order one."""
+    zone = meshgen.uniform_zone(12, order="rowmajor", boundary=meshgen.INFLOW, x_min=0.0, x_max=1.0, y_min=0.0, y_max=1.0)
+    K = 144
+
+    def after(mesh):
+        mesh.initial_conditions()
+        return ndg.Solver2D_t.run(mesh, steps, 0.1)
+
+    a, b = (ndg.Mesh2D_t(zone, N, maximum_N=N + 2) for _ in range(2))
+    dt = ndg.Solver2D_t.get_delta_t(a)
+
+    def compare(t, m, n):
+        a.time_stage(m, n)
+        for _ in range(n):
+            ndg.Solver2D_t.stage(b, m, t, dt)
+        assert np.array_equal(_get(a), _get(b)), (m, n)
+
+    t = after(a)
+    assert after(b) == t
+    for m, n in ((1, 3), (2, 4), (0, 1)):
+        compare(t, m, n)
+    ndg.Solver2D_t.stage(a, 1, t + 0.3, dt)
+    ndg.Solver2D_t.stage(b, 1, t + 0.3, dt)
+    compare(t + 0.3, 1, 2)
+    a.autotune(3)
+    a.set_tile(0)
+    compare(t + 0.3, 1, 3)
+    t = after(a)
+    after(b)
+    for mesh in (a, b):
+        mesh.adapt((np.arange(K) % 3 == 0).astype(np.int32), np.full(K, 2.0))
+    compare(t, 1, 2)
+    for mesh in (a, b):
+        mesh.close()
