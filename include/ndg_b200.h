@@ -268,11 +268,15 @@ ndg_status ndg_time_stage(ndg_ctx* ctx, int32_t m, int32_t n_launches, double* a
 ndg_status ndg_autotune(ndg_ctx* ctx, int32_t n_launches, int32_t* elements_per_block, double* best_ms);
 /* Sets the tile of the current form by hand (0 = the default). */
 ndg_status ndg_set_tile(ndg_ctx* ctx, int32_t elements_per_block);
-/* The candidate tiles of the loaded order and current form, and the default
- * tile of the kernel with three threads per element line (the one that runs
- * with ndg_ctx_keep_derivative). The kernel with one thread per line, which
- * runs most orders, has a default of its own: 16 elements up to order 10. */
+/* The candidate tiles of the kernel that runs the loaded mesh in the current
+ * form, and its default tile. The kernel with one thread per element line runs
+ * most meshes; with ndg_ctx_keep_derivative the one with three threads per line
+ * does, and switching between them keeps a tile both have (else the default). */
 ndg_status ndg_tile_candidates(const ndg_ctx* ctx, int32_t* out, int32_t capacity, int32_t* count, int32_t* default_tile);
+/* The name of the stage kernel that the next stage launches on a mesh of one
+ * order, with its order, form and tile (0: the default tile), as a profiler
+ * shows it without its argument type. */
+ndg_status ndg_stage_kernel(const ndg_ctx* ctx, char* out, int32_t capacity);
 
 /* No counterpart in the reference. Host wall time of the last adaptation
  * (ndg_adapt or ndg_adapt_flags) by phase, in ms: ms[0] the decisions and

@@ -124,6 +124,7 @@ def lib() -> C.CDLL:
         "ndg_delta_t_from_device": ([vp, vp, i64, dbl, vp, C.POINTER(dbl)], C.c_int),
         "ndg_autotune": ([vp, i32, C.POINTER(i32), C.POINTER(dbl)], C.c_int),
         "ndg_set_tile": ([vp, i32], C.c_int),
+        "ndg_stage_kernel": ([vp, vp, i32], C.c_int),
         "ndg_tile_candidates": ([vp, vp, i32, C.POINTER(i32), C.POINTER(i32)], C.c_int),
         "ndg_adjoint_create": ([vp, i32, vp, C.POINTER(vp)], C.c_int),
         "ndg_adjoint_destroy": ([vp], C.c_int),
@@ -382,6 +383,12 @@ class Mesh2D_t:
         n, d = C.c_int32(), C.c_int32()
         _check(lib().ndg_tile_candidates(self._ctx.h, C.cast(out, C.c_void_p), 16, C.byref(n), C.byref(d)))
         return list(out[:n.value]), d.value
+
+    def stage_kernel(self) -> str:
+        """Name of the kernel the next stage launches (meshes of one order)."""
+        buf = C.create_string_buffer(96)
+        _check(lib().ndg_stage_kernel(self._ctx.h, buf, len(buf)))
+        return buf.value.decode()
 
     def launches(self) -> int:
         n = C.c_int64()

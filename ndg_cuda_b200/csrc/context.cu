@@ -202,33 +202,38 @@ cudaError_t issue_general_stage(ndg_ctx* c, int m, int in) {
     return err;
 }
 
-// Whether the uniform stage runs the line kernel (line_stage.cuh): on a mesh
-// of its orders and sizes, in the default and FP32 forms, with its own tiles.
-// The time derivative (keep_derivative) is a by-product only of the
-// three-threads-a-line kernel, which also runs where a periodic seam's two
-// normals are not opposite.
-bool line_mesh(const ndg_ctx* c) { return !c->general && c->seams_opposite && dev::line_kernel_runs(c->N, fp32(c), c->K * c->n_instances); }
-bool line_stage(const ndg_ctx* c) {
-    return line_mesh(c) && !strict(c) && !c->keep_derivative && c->tile[fp32(c) ? 1 : 0] < dev::kTensorTile;
+// Whether the uniform stage of a form (FP64 default rounding, or FP32) runs the
+// line kernel (line_stage.cuh): on a mesh of its orders and sizes. The time
+// derivative (keep_derivative) is a by-product only of the three-threads-a-line
+// kernel, which also runs where a periodic seam's two normals are not opposite.
+bool line_form(const ndg_ctx* c, bool f32) {
+    return !c->general && c->seams_opposite && !c->keep_derivative && dev::line_kernel_runs(c->N, f32, c->K * c->n_instances);
 }
-// Whether the tile codes below kTensorTile are the line kernel's.
-bool line_tiles(const ndg_ctx* c) { return line_mesh(c) || dev::line_kernel_always(c->N); }
+
+// The kernel of the context's uniform stage: the one that runs a tile code
+// belongs to (tile_candidates lists that kernel's, and the tensor-core ones).
+enum class StageKernel { line, tile, standard };
+StageKernel stage_kernel(const ndg_ctx* c) {
+    if (strict(c)) return StageKernel::standard;
+    const int tile = c->tile[fp32(c) ? 1 : 0];
+    if (tile < dev::kTensorTile && line_form(c, fp32(c))) return StageKernel::line;
+    return tile ? StageKernel::tile : StageKernel::standard;
+}
+bool line_stage(const ndg_ctx* c) { return stage_kernel(c) == StageKernel::line; }
 
 // One stage. The step state is in step buffer `sp` (mixed-order meshes keep it
 // in buffer 0 and end a step by a launch of their own).
 cudaError_t issue_stage(ndg_ctx* c, int m, int in, int sp, bool advance) {
     if (c->general) return issue_general_stage(c, m, in);
-    if (line_stage(c))
-        return fp32(c) ? dev::launch_line_fp32(c->N, c->tile[1], stage_args(c, m, in, sp, advance), c->stream)
-                       : dev::launch_line_fp64(c->N, c->tile[0], stage_args(c, m, in, sp, advance), c->stream);
-    const int tile = c->tile[fp32(c) ? 1 : 0];
-    const bool variant = tile >= dev::kTensorTile || !line_tiles(c);
-    if (fp32(c)) {
-        if (tile && variant) return dev::launch_stage_variant_fp32(c->N, c->tile[1], stage_args(c, m, in, sp, advance), c->stream);
-        return dev::launch_stage_f32(c->N, stage_args(c, m, in, sp, advance), c->stream);
+    const dev::StageArgs a = stage_args(c, m, in, sp, advance);
+    const bool f32 = fp32(c);
+    const int tile = c->tile[f32 ? 1 : 0];
+    switch (stage_kernel(c)) {
+        case StageKernel::line: return f32 ? dev::launch_line_fp32(c->N, tile, a, c->stream) : dev::launch_line_fp64(c->N, tile, a, c->stream);
+        case StageKernel::tile:
+            return f32 ? dev::launch_stage_variant_fp32(c->N, tile, a, c->stream) : dev::launch_stage_variant_fp64(c->N, tile, a, c->stream);
+        default: return f32 ? dev::launch_stage_f32(c->N, a, c->stream) : dev::launch_stage(c->N, strict(c), a, c->stream);
     }
-    if (!strict(c) && tile && variant) return dev::launch_stage_variant_fp64(c->N, c->tile[0], stage_args(c, m, in, sp, advance), c->stream);
-    return dev::launch_stage(c->N, strict(c), stage_args(c, m, in, sp, advance), c->stream);
 }
 
 // The FP32 form on a mixed-order mesh allocates its trace buffers the first
@@ -258,21 +263,24 @@ void launch_stage(ndg_ctx* c, int m) {
     c->launches += c->general ? general_stage_launches(c) : 1;
 }
 
-// The tile candidates of the context's form (FP64 or FP32).
-std::vector<int> tile_candidates(const ndg_ctx* c) {
+// The tile candidates of a form (FP64 or FP32).
+std::vector<int> tile_candidates(const ndg_ctx* c, bool f32) {
     int buf[16];
-    const int n = fp32(c) ? dev::tile_candidates_fp32(c->N, line_tiles(c), buf, 16) : dev::tile_candidates_fp64(c->N, line_tiles(c), buf, 16);
+    const bool line = line_form(c, f32);
+    const int n = f32 ? dev::tile_candidates_fp32(c->N, line, buf, 16) : dev::tile_candidates_fp64(c->N, line, buf, 16);
     return std::vector<int>(buf, buf + n);
 }
 
-void set_tile(ndg_ctx* c, int epb) {
+bool set_tile(ndg_ctx* c, bool f32, int epb) {
     if (epb != 0) {
-        const std::vector<int> cand = tile_candidates(c);
-        if (std::find(cand.begin(), cand.end(), epb) == cand.end()) fail(NDG_ERR_INVALID_ARG, "not a candidate tile of this order and form");
-        check_cuda(fp32(c) ? dev::prepare_stage_variant_fp32(c->N, line_tiles(c), epb) : dev::prepare_stage_variant_fp64(c->N, line_tiles(c), epb), "kernel attributes");
+        const std::vector<int> cand = tile_candidates(c, f32);
+        if (std::find(cand.begin(), cand.end(), epb) == cand.end()) return false;
+        const bool line = line_form(c, f32);
+        check_cuda(f32 ? dev::prepare_stage_variant_fp32(c->N, line, epb) : dev::prepare_stage_variant_fp64(c->N, line, epb), "kernel attributes");
     }
-    c->tile[fp32(c) ? 1 : 0] = epb;
+    c->tile[f32 ? 1 : 0] = epb;
     drop_graphs(c);
+    return true;
 }
 
 void ensure_traces(ndg_ctx* c) {
@@ -1120,6 +1128,10 @@ ndg_status ndg_ctx_keep_derivative(ndg_ctx* ctx, int32_t enable) {
         make_current(ctx);
         ctx->keep_derivative = enable != 0;
         drop_graphs(ctx);
+        // Another kernel may run from here: a tile stays where that one has it.
+        if (ctx->has_mesh && ctx->device >= 0 && !ctx->general)
+            for (bool f32 : {false, true})
+                if (!set_tile(ctx, f32, ctx->tile[f32 ? 1 : 0])) ctx->tile[f32 ? 1 : 0] = 0;
         if (ctx->has_mesh && ctx->device >= 0) {
             if (ctx->keep_derivative) {
                 ctx->G.allocate(static_cast<size_t>(3 * ctx->block * ctx->n_instances));
@@ -1502,13 +1514,38 @@ ndg_status ndg_tile_candidates(const ndg_ctx* ctx, int32_t* out, int32_t capacit
     return guarded([&] {
         require_mesh(ctx);
         if (ctx->general) fail(NDG_ERR_UNSUPPORTED, "tiles are tuned for meshes of one order");
-        const std::vector<int> cand = tile_candidates(ctx);
+        const std::vector<int> cand = tile_candidates(ctx, fp32(ctx));
         if (count) *count = static_cast<int32_t>(cand.size());
         if (out) {
             if (capacity < static_cast<int32_t>(cand.size())) fail(NDG_ERR_INVALID_ARG, "output buffer too small");
             std::copy(cand.begin(), cand.end(), out);
         }
-        if (default_tile) *default_tile = dev::elements_per_block(ctx->N);
+        if (default_tile) *default_tile = !strict(ctx) && line_form(ctx, fp32(ctx)) ? dev::line_default_tile(ctx->N) : dev::elements_per_block(ctx->N);
+    });
+}
+
+ndg_status ndg_stage_kernel(const ndg_ctx* ctx, char* out, int32_t capacity) {
+    return guarded([&] {
+        require_mesh(ctx);
+        if (!out) fail(NDG_ERR_INVALID_ARG, "out is NULL");
+        if (ctx->general) fail(NDG_ERR_UNSUPPORTED, "a mesh of several orders runs one kernel per order group");
+        const bool f32 = fp32(ctx);
+        const int tile = ctx->tile[f32 ? 1 : 0];
+        const std::string N = std::to_string(ctx->N);
+        std::string name;
+        switch (stage_kernel(ctx)) {
+            case StageKernel::line:
+                name = "line_stage_kernel<" + N + (f32 ? ", float, " : ", double, ") + std::to_string(tile ? tile : dev::line_default_tile(ctx->N)) + ">";
+                break;
+            case StageKernel::tile: {
+                const std::string form = std::to_string(tile % dev::kTensorTile) + (tile >= dev::kTensorTile ? ", true>" : ", false>");
+                name = f32 ? "stage_kernel_f32<" + N + ", " + form : "stage_kernel<" + N + ", false, " + form;
+                break;
+            }
+            default: name = f32 ? "stage_kernel_f32<" + N + ", 0, false>" : "stage_kernel<" + N + (strict(ctx) ? ", true" : ", false") + ", 0, false>";
+        }
+        if (capacity < static_cast<int32_t>(name.size() + 1)) fail(NDG_ERR_INVALID_ARG, "output buffer too small");
+        std::memcpy(out, name.c_str(), name.size() + 1);
     });
 }
 
@@ -1519,7 +1556,7 @@ ndg_status ndg_set_tile(ndg_ctx* ctx, int32_t elements_per_block) {
         if (ctx->general) fail(NDG_ERR_UNSUPPORTED, "tiles are tuned for meshes of one order");
         if (strict(ctx) && elements_per_block != 0) fail(NDG_ERR_UNSUPPORTED, "the strict form keeps its default tile");
         make_current(ctx);
-        set_tile(ctx, elements_per_block);
+        if (!set_tile(ctx, fp32(ctx), elements_per_block)) fail(NDG_ERR_INVALID_ARG, "not a candidate tile of this order and form");
     });
 }
 
@@ -1529,7 +1566,7 @@ ndg_status ndg_autotune(ndg_ctx* ctx, int32_t n_launches, int32_t* elements_per_
         require_device(ctx);
         if (n_launches < 1) fail(NDG_ERR_INVALID_ARG, "n_launches must be >= 1");
         make_current(ctx);
-        const int form = fp32(ctx) ? 1 : 0;
+        const bool f32 = fp32(ctx);
         if (ctx->general || strict(ctx)) {
             // mixed-order meshes and the strict form keep their tiles
             if (elements_per_block) *elements_per_block = 0;
@@ -1543,7 +1580,7 @@ ndg_status ndg_autotune(ndg_ctx* ctx, int32_t n_launches, int32_t* elements_per_
         k0.allocate(values);
         check_cuda(cudaMemcpyAsync(q0.ptr, ctx->q.ptr, values * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream), "state copy");
         check_cuda(cudaMemcpyAsync(k0.ptr, ctx->k.ptr, values * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream), "state copy");
-        std::vector<int> cand = tile_candidates(ctx);
+        std::vector<int> cand = tile_candidates(ctx, f32);
         cand.insert(cand.begin(), 0);  // the default tile
         hold_step(ctx);
         cudaEvent_t e0, e1;
@@ -1552,7 +1589,7 @@ ndg_status ndg_autotune(ndg_ctx* ctx, int32_t n_launches, int32_t* elements_per_
         int best = 0;
         double best_t = INFINITY;
         for (int epb : cand) {
-            set_tile(ctx, epb);
+            set_tile(ctx, f32, epb);
             ensure_traces(ctx);
             launch_stage(ctx, 1);  // warm-up
             check_cuda(cudaEventRecord(e0, ctx->stream), "cudaEventRecord");
@@ -1574,8 +1611,7 @@ ndg_status ndg_autotune(ndg_ctx* ctx, int32_t n_launches, int32_t* elements_per_
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
         check_device_error(ctx);
-        set_tile(ctx, best);
-        ctx->tile[form] = best;
+        set_tile(ctx, f32, best);
         check_cuda(cudaStreamSynchronize(ctx->stream), "autotune");
         if (elements_per_block) *elements_per_block = best;
         if (best_ms) *best_ms = best_t;

@@ -87,7 +87,7 @@ int candidates(int* out, int max) {
 
 }  // namespace
 
-bool line_kernel_always(int N) { return line_every_size(N); }
+int line_default_tile(int N) { return line_default_elements(N); }
 
 bool line_kernel_runs(int N, bool fp32, int64_t elements) {
     return line_order(N, fp32) && (line_every_size(N) || elements >= kLineMinElements);

@@ -86,7 +86,7 @@ cudaError_t launch_stage_variant_fp32(int N, int epb, const StageArgs& a, cudaSt
 // outgoing characteristic per side node, [instance][field_stride][side][N+1]
 // in the far slots, at the start of the trace buffers.
 bool line_kernel_runs(int N, bool fp32, int64_t elements);  // elements of all instances
-bool line_kernel_always(int N);                             // at every size: no three-threads-a-line tiles are compiled
+int line_default_tile(int N);
 int line_candidates_fp64(int N, int* out, int max);
 int line_candidates_fp32(int N, int* out, int max);
 cudaError_t prepare_line_fp64(int N, int elements);

@@ -27,8 +27,7 @@ constexpr int kTensorMinOrder = 6;
 template <bool F32, int N, int E, bool TC = false>
 struct Variant {
     using T = std::conditional_t<F32, TileF<N, E>, Tile<N, E>>;
-    // Orders that run the line kernel at every size have no SIMT tiles.
-    static constexpr bool feasible = T::kThreads <= 512 && T::kBytes <= 113 * 1024 && (TC ? E <= 8 && N >= kTensorMinOrder : !line_every_size(N));
+    static constexpr bool feasible = T::kThreads <= 512 && T::kBytes <= 113 * 1024 && (!TC || (E <= 8 && N >= kTensorMinOrder));
 };
 
 template <int N>

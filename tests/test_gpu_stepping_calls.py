@@ -120,3 +120,76 @@ def test_timed_stages_run_at_the_state_the_last_call_left(N, steps):
     compare(t, 1, 2)
     for mesh in (a, b):
         mesh.close()
+
+
+def _launched(mesh, steps=1):
+    """Names of the stage kernels a run launches, as CUPTI records them."""
+    from torch.profiler import ProfilerActivity, profile
+    ndg.Solver2D_t.run(mesh, steps)
+    mesh.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        ndg.Solver2D_t.run(mesh, steps)
+        mesh.synchronize()
+    names = [e.name for e in prof.events() if "stage_kernel" in e.name]
+    return {n.replace("void ", "").replace("ndg::dev::", "").split("(")[0] for n in names}
+
+
+def _is(name, launched):
+    """stage_kernel() leaves out the line kernel's argument type."""
+    return len(launched) == 1 and (launched == {name} or next(iter(launched)).startswith(name[:-1] + ", "))
+
+
+@pytest.mark.parametrize("precision", [ndg.FP64, ndg.FP32])
+@pytest.mark.parametrize("N,res", [(3, 8), (6, 40), (6, 8), (8, 40), (10, 40)])
+def test_tiles_are_those_of_the_kernel_that_runs(N, res, precision):
+    """With keep_derivative the three-threads-a-line kernel runs, so its tiles
+    are the candidates and take effect; without, the line kernel's where it
+    runs. Switching keeps a tile that both kernels have, and the fields do not
+    depend on any of it beyond rounding (4 steps; the bounds of
+    tests/test_gpu_line_stage.py)."""
+    tol = 1e-13 if precision == ndg.FP64 else 2e-6
+    mesh = ndg.Mesh2D_t(meshgen.uniform_zone(res, boundary=meshgen.WALL, jitter=0.1, seed=2, order="rowmajor"), N, precision=precision)
+    rng = np.random.default_rng(N)
+    start = [rng.standard_normal(mesh.field_size) for _ in FIELDS]
+
+    def fields():
+        for f, v in zip(FIELDS, start):
+            mesh.set_field(f, v)
+        ndg.Solver2D_t.run(mesh, 4)
+        return _get(mesh)
+
+    reference = fields()
+    line = N <= 4 or res >= 40
+    assert mesh.stage_kernel().startswith("line_stage_kernel" if line else "stage_kernel")
+    seen = {}
+    for keep in (1, 0, 1):
+        assert ndg.lib().ndg_ctx_keep_derivative(mesh.handle, keep) == 0
+        candidates, default = mesh.tile_candidates()
+        mesh.set_tile(0)
+        names = {mesh.stage_kernel()}
+        for tile in candidates:
+            mesh.set_tile(tile)
+            name = mesh.stage_kernel()
+            names.add(name)
+            assert name.startswith("line_") == (line and not keep and tile < ndg.TENSOR_TILE), (keep, tile, name)
+            assert _is(name, _launched(mesh)), (keep, tile, name)
+            got = fields()
+            assert np.linalg.norm(got - reference) <= tol * np.linalg.norm(reference), (keep, tile)
+        assert len(names) >= len(candidates)  # every tile is a kernel of its own; the default may be one of them
+        assert default > 0
+        seen[keep] = candidates
+    assert set(seen[1]) <= set(seen[0])
+    # 4 elements: a tile of both kernels; 16 at order 10: only the line kernel's
+    mesh.set_tile(4)
+    assert ndg.lib().ndg_ctx_keep_derivative(mesh.handle, 0) == 0
+    assert ", 4" in mesh.stage_kernel()
+    extra = sorted(set(seen[0]) - set(seen[1]))
+    if extra:
+        mesh.set_tile(extra[-1])
+        assert ndg.lib().ndg_ctx_keep_derivative(mesh.handle, 1) == 0
+        assert ", 0, false>" in mesh.stage_kernel()
+    got = fields()
+    assert np.linalg.norm(got - reference) <= tol * np.linalg.norm(reference)
+    tile, ms = mesh.autotune(3)
+    assert ms > 0 and (tile == 0 or tile in mesh.tile_candidates()[0])
+    mesh.close()
