@@ -109,15 +109,16 @@ cudaError_t prepare_speed_kernels(int N, bool fp32);
 cudaError_t launch_speed_stage(int N, bool fp32, const SpeedStageArgs& a, cudaStream_t stream);
 // The same stage by the line kernel (line_stage.cuh; where line_kernel_runs):
 // trace_in / trace_out then hold its characteristics (launch_line_traces_*),
-// and G_out is not written (with first set, k is G).
-cudaError_t prepare_speed_line(int N, bool fp32);
-cudaError_t launch_speed_line(int N, bool fp32, const SpeedStageArgs& a, cudaStream_t stream);
+// and G_out is not written (with first set, k is G). seam: of a mesh with
+// kSeamNormal sides.
+cudaError_t prepare_speed_line(int N, bool fp32, bool seam);
+cudaError_t launch_speed_line(int N, bool fp32, bool seam, const SpeedStageArgs& a, cudaStream_t stream);
 cudaError_t launch_adjoint_stage(int N, bool fp32, const AdjointStageArgs& a, cudaStream_t stream);
 // The same stage with one thread per line (adjoint_line.cu; where
 // line_kernel_runs): atr_in / atr_out then hold one scalar per side node in
 // the receiving side's far slots, [Kp][side][N+1].
-cudaError_t prepare_adjoint_line(int N, bool fp32);
-cudaError_t launch_adjoint_line(int N, bool fp32, const AdjointStageArgs& a, cudaStream_t stream);
+cudaError_t prepare_adjoint_line(int N, bool fp32, bool seam);
+cudaError_t launch_adjoint_line(int N, bool fp32, bool seam, const AdjointStageArgs& a, cudaStream_t stream);
 // grad_c[e] = acc[e][0] + sum over sides of acc[e][1+s] (boundary sides) or
 // (acc[e][1+s] + acc[nb][1+s']) / 2 (sides shared with element nb, side s').
 cudaError_t launch_speed_gradient(const double* acc, const int2* link, int64_t K, double* grad_c, cudaStream_t stream);

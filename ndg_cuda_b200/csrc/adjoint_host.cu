@@ -38,7 +38,7 @@ struct ndg_adjoint {
     bool fp32 = false;
     // The forward and adjoint stages run the line kernels in this form (by the
     // rule of the uniform stage), with one value per side node in tr and atr.
-    bool line() const { return ctx->seams_opposite && ndg::dev::line_kernel_runs(N, fp32, K); }
+    bool line() const { return ndg::dev::line_kernel_runs(N, fp32, K); }
     ndg::dev::Receivers rec{};
     // the last forward
     bool has_forward = false;
@@ -142,7 +142,7 @@ dev::SpeedStageArgs speed_args(ndg_adjoint* a, int m, int in, double dt) {
 }
 
 cudaError_t launch_speed(ndg_adjoint* a, const dev::SpeedStageArgs& s, cudaStream_t stream) {
-    return a->line() ? dev::launch_speed_line(a->N, a->fp32, s, stream) : dev::launch_speed_stage(a->N, a->fp32, s, stream);
+    return a->line() ? dev::launch_speed_line(a->N, a->fp32, a->ctx->seam_normals, s, stream) : dev::launch_speed_stage(a->N, a->fp32, s, stream);
 }
 
 dev::AdjointStageArgs adjoint_args(ndg_adjoint* a, int in) {
@@ -168,7 +168,7 @@ dev::AdjointStageArgs adjoint_args(ndg_adjoint* a, int in) {
 }
 
 cudaError_t launch_adjoint(ndg_adjoint* a, const dev::AdjointStageArgs& s, cudaStream_t stream) {
-    return a->line() ? dev::launch_adjoint_line(a->N, a->fp32, s, stream) : dev::launch_adjoint_stage(a->N, a->fp32, s, stream);
+    return a->line() ? dev::launch_adjoint_line(a->N, a->fp32, a->ctx->seam_normals, s, stream) : dev::launch_adjoint_stage(a->N, a->fp32, s, stream);
 }
 
 void launch_traces_of_q(ndg_adjoint* a, int out, cudaStream_t stream = nullptr) {
@@ -319,8 +319,8 @@ ndg_status ndg_adjoint_create(ndg_ctx* ctx, int32_t n_receivers, const double* r
         check_cuda(dev::prepare_kernels_f32(a->N), "kernel attributes");
         for (bool f32 : {false, true})
             if (dev::line_kernel_runs(a->N, f32, a->K)) {
-                check_cuda(dev::prepare_speed_line(a->N, f32), "kernel attributes");
-                check_cuda(dev::prepare_adjoint_line(a->N, f32), "kernel attributes");
+                check_cuda(dev::prepare_speed_line(a->N, f32, ctx->seam_normals), "kernel attributes");
+                check_cuda(dev::prepare_adjoint_line(a->N, f32, ctx->seam_normals), "kernel attributes");
             }
         check_cuda(cudaEventCreate(&a->ev[0]), "event");
         check_cuda(cudaEventCreate(&a->ev[1]), "event");

@@ -12,7 +12,9 @@
 // With b = (n . psi_uv - psi_p) / 2 and a = (n . psi_uv + psi_p) / 2 of a
 // side's flux adjoint psi (n outward), the transposed upwind flux is a (1, n)
 // on the own trace and b (1, -n) on the far one, so sides exchange the scalar
-// b: a third of the trace traffic of three components, as in the forward.
+// b: a third of the trace traffic of three components, as in the forward. The
+// receiving element applies the sender's normal: the opposite of its own, or on
+// a seam (kSeamNormal) the neighbour side's.
 //
 // Measured, backward of 60 steps with checkpoints every 20 at 96 x 96 (its
 // recomputation included), ms, against three threads a line: FP64 N = 4 2.00
@@ -70,7 +72,7 @@ struct AdjLineTile {
     static constexpr bool feasible = kBytes <= 226 * 1024;
 };
 
-template <int N, typename R, int E>
+template <int N, typename R, int E, bool Seam>
 __global__ void __launch_bounds__(AdjLineTile<N, R, E>::kThreads, AdjLineTile<N, R, E>::kMinBlocks)
     adjoint_line_kernel(AdjointStageArgs a, const __grid_constant__ AdjLineCoeffs<N, R> cf) {
     using A = AdjLineTile<N, R, E>;
@@ -132,7 +134,7 @@ __global__ void __launch_bounds__(AdjLineTile<N, R, E>::kThreads, AdjLineTile<N,
         side[16 * E + o] = dx;
         side[20 * E + o] = dy;
         side[24 * E + o] = (kind == kMirror || kind == kCopy) ? R(a.gscale[o4]) : R(0);
-        to_s[o] = kind == kInterior ? (lk.x * 4 + (lk.y & 3)) : ~kind;
+        to_s[o] = side_entry<Seam>(lk);
     }
     for (int i = tid; i < E; i += A::kThreads) rmask[i] = 0ull;
     const R ce = active ? R(a.c[ge]) : R(1);
@@ -208,7 +210,7 @@ __global__ void __launch_bounds__(AdjLineTile<N, R, E>::kThreads, AdjLineTile<N,
         const R av = hn + hp, b = hn - hp;
         R tp = av, tn = av;
         const int to = to_s[s * E + e];
-        if (to >= 0) {
+        if (side_interior<Seam>(to)) {
             const R f = far_s[e * SE + s * n + idx];
             tp += f;
             tn += f;
@@ -220,14 +222,22 @@ __global__ void __launch_bounds__(AdjLineTile<N, R, E>::kThreads, AdjLineTile<N,
         t[0] = tp;
         t[1] = tn * nx;
         t[2] = tn * ny;
+        if constexpr (Seam) {
+            if (to < 0 && side_interior<Seam>(to)) {
+                const double2 fn = far_inward(side_far<Seam>(to), a.normal, a.link);
+                const R f = far_s[e * SE + s * n + idx];
+                t[1] = fma(f, R(fn.x), av * nx);
+                t[2] = fma(f, R(fn.y), av * ny);
+            }
+        }
         return (own[0] * t[0] + own[1] * t[1] + own[2] * t[2]) / side[12 * E + s * E + e];
     };
     const auto publish = [&](int s, int idx, const R (&l)[3]) {
         const int to = to_s[s * E + e];
-        if (to < 0) return;
+        if (!side_interior<Seam>(to)) return;
         R hp, hn;
         halves(s, l, hp, hn);
-        atr_out[static_cast<int64_t>(to) * n + (N - idx)] = hn - hp;
+        atr_out[side_far<Seam>(to) * n + (N - idx)] = hn - hp;
     };
     // Volume part of the speed derivative on this thread's column and row: in
     // the FP32 form one FP32 sum per field, joined in FP64. One sum over the
@@ -408,11 +418,11 @@ constexpr int elements() {
 }
 
 template <int N, typename R>
-cudaError_t prepare() {
+cudaError_t prepare(bool seam) {
     if constexpr (line_order(N, sizeof(R) == 4)) {
         constexpr int E = elements<N>();
         static_assert(AdjLineTile<N, R, E>::feasible);
-        return cudaFuncSetAttribute(adjoint_line_kernel<N, R, E>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        return cudaFuncSetAttribute(seam ? adjoint_line_kernel<N, R, E, true> : adjoint_line_kernel<N, R, E, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     static_cast<int>(AdjLineTile<N, R, E>::kBytes));
     } else {
         return cudaErrorInvalidValue;
@@ -420,11 +430,11 @@ cudaError_t prepare() {
 }
 
 template <int N, typename R>
-cudaError_t launch(const AdjointStageArgs& a, cudaStream_t stream) {
+cudaError_t launch(bool seam, const AdjointStageArgs& a, cudaStream_t stream) {
     if constexpr (line_order(N, sizeof(R) == 4)) {
         constexpr int E = elements<N>();
         using A = AdjLineTile<N, R, E>;
-        return launch_dependent(adjoint_line_kernel<N, R, E>, dim3(static_cast<unsigned>((a.n_elements + E - 1) / E)), A::kThreads, A::kBytes, stream, a,
+        return launch_dependent(seam ? adjoint_line_kernel<N, R, E, true> : adjoint_line_kernel<N, R, E, false>, dim3(static_cast<unsigned>((a.n_elements + E - 1) / E)), A::kThreads, A::kBytes, stream, a,
                                 make_adj_line_coeffs<N, R>());
     } else {
         return cudaErrorInvalidValue;
@@ -450,9 +460,11 @@ cudaError_t launch(const AdjointStageArgs& a, cudaStream_t stream) {
         default: return cudaErrorInvalidValue;                                          \
     }
 
-cudaError_t prepare_adjoint_line(int N, bool fp32) { NDG_ADJOINT_LINE_DISPATCH(prepare) }
+cudaError_t prepare_adjoint_line(int N, bool fp32, bool seam) { NDG_ADJOINT_LINE_DISPATCH(prepare, seam) }
 
-cudaError_t launch_adjoint_line(int N, bool fp32, const AdjointStageArgs& a, cudaStream_t stream) { NDG_ADJOINT_LINE_DISPATCH(launch, a, stream) }
+cudaError_t launch_adjoint_line(int N, bool fp32, bool seam, const AdjointStageArgs& a, cudaStream_t stream) {
+    NDG_ADJOINT_LINE_DISPATCH(launch, seam, a, stream)
+}
 
 }  // namespace dev
 }  // namespace ndg

@@ -205,9 +205,9 @@ cudaError_t issue_general_stage(ndg_ctx* c, int m, int in) {
 // Whether the uniform stage of a form (FP64 default rounding, or FP32) runs the
 // line kernel (line_stage.cuh): on a mesh of its orders and sizes. The time
 // derivative (keep_derivative) is a by-product only of the three-threads-a-line
-// kernel, which also runs where a periodic seam's two normals are not opposite.
+// kernel.
 bool line_form(const ndg_ctx* c, bool f32) {
-    return !c->general && c->seams_opposite && !c->keep_derivative && dev::line_kernel_runs(c->N, f32, c->K * c->n_instances);
+    return !c->general && !c->keep_derivative && dev::line_kernel_runs(c->N, f32, c->K * c->n_instances);
 }
 
 // The kernel of the context's uniform stage: the one that runs a tile code
@@ -229,7 +229,7 @@ cudaError_t issue_stage(ndg_ctx* c, int m, int in, int sp, bool advance) {
     const bool f32 = fp32(c);
     const int tile = c->tile[f32 ? 1 : 0];
     switch (stage_kernel(c)) {
-        case StageKernel::line: return f32 ? dev::launch_line_fp32(c->N, tile, a, c->stream) : dev::launch_line_fp64(c->N, tile, a, c->stream);
+        case StageKernel::line: return f32 ? dev::launch_line_fp32(c->N, c->seam_normals, tile, a, c->stream) : dev::launch_line_fp64(c->N, c->seam_normals, tile, a, c->stream);
         case StageKernel::tile:
             return f32 ? dev::launch_stage_variant_fp32(c->N, tile, a, c->stream) : dev::launch_stage_variant_fp64(c->N, tile, a, c->stream);
         default: return f32 ? dev::launch_stage_f32(c->N, a, c->stream) : dev::launch_stage(c->N, strict(c), a, c->stream);
@@ -275,8 +275,10 @@ bool set_tile(ndg_ctx* c, bool f32, int epb) {
     if (epb != 0) {
         const std::vector<int> cand = tile_candidates(c, f32);
         if (std::find(cand.begin(), cand.end(), epb) == cand.end()) return false;
-        const bool line = line_form(c, f32);
-        check_cuda(f32 ? dev::prepare_stage_variant_fp32(c->N, line, epb) : dev::prepare_stage_variant_fp64(c->N, line, epb), "kernel attributes");
+        if (epb < dev::kTensorTile && line_form(c, f32))
+            check_cuda(f32 ? dev::prepare_line_fp32(c->N, c->seam_normals, epb) : dev::prepare_line_fp64(c->N, c->seam_normals, epb), "kernel attributes");
+        else
+            check_cuda(f32 ? dev::prepare_stage_variant_fp32(c->N, epb) : dev::prepare_stage_variant_fp64(c->N, epb), "kernel attributes");
     }
     c->tile[f32 ? 1 : 0] = epb;
     drop_graphs(c);
@@ -311,7 +313,7 @@ void ensure_traces(ndg_ctx* c) {
             if (t.count != count) t.allocate(count);
         a.trace_out_f = c->tr32[c->cur].ptr;
         check_cuda(dev::prepare_kernels_f32(c->N), "kernel attributes");
-        if (line) check_cuda(dev::prepare_line_fp32(c->N, 0), "kernel attributes");
+        if (line) check_cuda(dev::prepare_line_fp32(c->N, c->seam_normals, 0), "kernel attributes");
         check_cuda(line ? dev::launch_line_traces_fp32(c->N, a, c->stream) : dev::launch_traces_f32(c->N, a, c->stream), "trace kernel launch");
     } else if (line) {
         check_cuda(dev::launch_line_traces_fp64(c->N, a, c->stream), "trace kernel launch");
@@ -471,17 +473,8 @@ void upload_plan(ndg_ctx* c, const Layout& l) {
     if (!l.general) {
         if (c->N > kMaxOrder) fail(NDG_ERR_UNSUPPORTED, "orders above 16 have no compiled kernel");
         SidePlan plan = build_side_plan(c->topo, c->tables);
-        // Outward normals n of the two sides of an interior link: opposite to
-        // rounding on every conforming face and on seams that are translates.
-        c->seams_opposite = true;
-        for (size_t i = 0; i < 4 * K && c->seams_opposite; ++i) {
-            const int32_t word = plan.link[2 * i + 1];
-            if (((word >> 2) & 7) != kInterior) continue;
-            const size_t o = 4 * static_cast<size_t>(plan.link[2 * i]) + static_cast<size_t>(word & 3);
-            const double s = ((word >> 5) & 1) == ((plan.link[2 * o + 1] >> 5) & 1) ? 1.0 : -1.0;
-            for (size_t d = 0; d < 2; ++d)
-                if (std::abs(plan.normal[2 * i + d] + s * plan.normal[2 * o + d]) > 1e-15) c->seams_opposite = false;
-        }
+        c->seam_normals = false;
+        for (size_t i = 0; i < 4 * K; ++i) c->seam_normals |= (plan.link[2 * i + 1] & kSeamNormal) != 0;
         // Tiles copy an even number of elements: pad the per-element arrays
         // to the even element count (the pad element has no sides).
         const size_t Kpad = static_cast<size_t>(c->Kp);
@@ -504,7 +497,7 @@ void upload_plan(ndg_ctx* c, const Layout& l) {
         c->tc32.upload(dev::tc_lane_table_fp32(c->N), c->stream);
         check_cuda(dev::prepare_kernels(c->N, false), "kernel attributes");
         check_cuda(dev::prepare_kernels(c->N, true), "kernel attributes");
-        if (dev::line_kernel_runs(c->N, false, c->K * c->n_instances)) check_cuda(dev::prepare_line_fp64(c->N, 0), "kernel attributes");
+        if (dev::line_kernel_runs(c->N, false, c->K * c->n_instances)) check_cuda(dev::prepare_line_fp64(c->N, c->seam_normals, 0), "kernel attributes");
         c->groups.clear();
         c->whole_groups.clear();
     } else {

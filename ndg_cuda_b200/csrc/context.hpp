@@ -111,8 +111,8 @@ struct ndg_ctx {
     bool has_error_estimate = false;
     int cur = 0;
     bool traces_valid = false;
-    bool line_traces = false;    // the traces hold the line kernel's characteristics
-    bool seams_opposite = true;  // both sides of every interior link have opposite normals (the line kernel's far slots need it)
+    bool line_traces = false;   // the traces hold the line kernel's characteristics
+    bool seam_normals = false;  // the mesh has kSeamNormal sides
     double dt_mesh = 0.0;
 
     // Mixed-order meshes (after adaptation) run the general stage path.

@@ -11,10 +11,11 @@
 //    256 x 256, FP64: 44.5 M warp instructions instead of 94.7 M and 12.7 M
 //    shared wavefronts instead of 25.5 M per launch.
 //  - The face flux reads the far side only through its outgoing
-//    characteristic w = p + (u, v) . n (n the far side's outward normal, the
-//    opposite of this side's), so sides exchange that one value per node
-//    instead of p, u and v: a third of the trace traffic and of the scattered
-//    stores. Far slots are [instance][element][side][node].
+//    characteristic w = p - (u, v) . n (n this side's outward normal), so sides
+//    exchange that one value per node instead of p, u and v: a third of the
+//    trace traffic and of the scattered stores. The sender takes its own normal
+//    for the opposite of n, or on a seam where it is not n itself (kSeamNormal).
+//    Far slots are [instance][element][side][node].
 //  - q and k arrive in shared memory together, ahead of the passes. With 16
 //    elements a tile and N + 1 odd the tile needs no padding (below): one bulk
 //    copy per field in, one out, issued by one thread.
@@ -45,6 +46,7 @@
 
 #include <cuda_runtime.h>
 
+#include <climits>
 #include <cstdint>
 #include <type_traits>
 
@@ -186,6 +188,34 @@ struct MLine {
     __device__ __forceinline__ MLine(R d0, R d1) : a(R(0.25) * (d0 + d1)), b(R(0.25) * (d1 - d0)) {}
     __device__ __forceinline__ R operator()(R t) const { return fma(t, b, a); }
 };
+
+// A side's entry in a tile's table of neighbours: the neighbour's side (element
+// 4 + side, below 2^31 - 16), or ~kind on a boundary. Seam (meshes that have a
+// seam whose two normals are not opposite, kSeamNormal): with the sign bit set
+// on those sides. Their far normal is read where it is used, by instantiations
+// of their own: in one kernel for all meshes a launch took 1 to 2% longer (N = 8,
+// 40 x 40 6.1 -> 6.8 us), and with every side's in the tile 1 to 7% (N = 8, 256 x
+// 256 93.8 -> 94.9 us, N = 12, 160 x 160 108 -> 115).
+template <bool Seam>
+__device__ __forceinline__ int side_entry(int2 lk) {
+    const int kind = (lk.y >> 2) & 7;
+    if (kind != kInterior) return ~kind;
+    const int far = lk.x * 4 + (lk.y & 3);
+    return Seam && (lk.y & kSeamNormal) ? far | INT_MIN : far;
+}
+template <bool Seam>
+__device__ __forceinline__ bool side_interior(int entry) {
+    return Seam ? static_cast<unsigned>(entry) < 0xfffffff0u : entry >= 0;
+}
+template <bool Seam>
+__device__ __forceinline__ int64_t side_far(int entry) {
+    return Seam ? entry & INT_MAX : entry;
+}
+// Minus the outward normal of the neighbour's side.
+__device__ __forceinline__ double2 far_inward(int64_t far, const double2* normal, const int2* link) {
+    const double2 nv = normal[far];
+    return ((link[far].y >> 5) & 1) ? nv : double2{-nv.x, -nv.y};
+}
 
 // The outgoing characteristic p + (u, v) . n, with fixed rounding: the stage
 // and the trace kernel must agree on it bit for bit.
@@ -342,7 +372,7 @@ __device__ __forceinline__ void line_product(const LineCoeffs<N, R>& cf, const R
 // adjoint module (adjoint.cuh: the volume term times the element's speed, the
 // face flux times the face's, optional copies of the stage input and of the
 // receivers' pressure; one instance, no inflow sides).
-template <int N, typename R, int E, typename Args>
+template <int N, typename R, int E, typename Args, bool Seam>
 __global__ void __launch_bounds__(LineTile<N, R, E>::kThreads, LineTile<N, R, E>::kMinBlocks) line_stage_kernel(Args a, const __grid_constant__ LineCoeffs<N, R> cf) {
     using T = LineTile<N, R, E>;
     constexpr int n = T::n, NN = T::NN, P = T::P, ES = T::ES, QS = T::QS, SE = T::SE;
@@ -354,7 +384,7 @@ __global__ void __launch_bounds__(LineTile<N, R, E>::kThreads, LineTile<N, R, E>
     R* rs = reinterpret_cast<R*>(bar + 2);
     R* far_s = rs + T::kFar;    // [element][SE] far characteristics
     R* side = rs + T::kSide;    // [nx, ny, edge metric, dx, dy][side][element]
-    int* to_s = reinterpret_cast<int*>(rs + T::kRs);  // [side][element] the neighbour's side (element 4 + side), or ~kind
+    int* to_s = reinterpret_cast<int*>(rs + T::kRs);  // [side][element] side_entry
     const int tid = threadIdx.x;
     const int64_t K = a.n_elements, Kp = a.field_stride;
     const int64_t e0 = static_cast<int64_t>(blockIdx.x) * E;
@@ -403,7 +433,6 @@ __global__ void __launch_bounds__(LineTile<N, R, E>::kThreads, LineTile<N, R, E>
     };
     const auto put_side = [&](int i, const SidePlanEntry& p) {
         const bool role = (p.lk.y >> 5) & 1;
-        const int kind = (p.lk.y >> 2) & 7;
         const R dx = R(p.c1.x - p.c0.x), dy = R(p.c1.y - p.c0.y);
         const int o = (i & 3) * E + (i >> 2);
         side[o] = R(role ? -p.nv.x : p.nv.x);
@@ -412,7 +441,7 @@ __global__ void __launch_bounds__(LineTile<N, R, E>::kThreads, LineTile<N, R, E>
         if constexpr (kSpeed) side[8 * E + o] *= R(p.speed);
         side[12 * E + o] = dx;
         side[16 * E + o] = dy;
-        to_s[o] = kind == kInterior ? (p.lk.x * 4 + (p.lk.y & 3)) : ~kind;
+        to_s[o] = side_entry<Seam>(p.lk);
     };
     SidePlanEntry first_side{};
     if (tid < 4 * ne) first_side = read_side(tid);
@@ -496,7 +525,7 @@ __global__ void __launch_bounds__(LineTile<N, R, E>::kThreads, LineTile<N, R, E>
         const R nx = side[s * E + e], ny = side[4 * E + s * E + e], sf = side[8 * E + s * E + e];
         const int to = to_s[s * E + e];
         R wR = far_s[e * SE + s * n + idx];
-        if (to < 0) {
+        if (!side_interior<Seam>(to)) {
             const int kind = ~to;
             R fp = R(0), fu = R(0), fv = R(0);
             if (kind == kMirror || kind == kCopy) {
@@ -532,7 +561,16 @@ __global__ void __launch_bounds__(LineTile<N, R, E>::kThreads, LineTile<N, R, E>
     // neighbour's far slot.
     const auto send = [&](int s, int idx, R p, R u, R v) {
         const int to = to_s[s * E + e];
-        if (to >= 0) tr_out[static_cast<int64_t>(to) * n + (N - idx)] = characteristic(p, u, v, side[s * E + e], side[4 * E + s * E + e]);
+        if (!side_interior<Seam>(to)) return;
+        R nx = side[s * E + e], ny = side[4 * E + s * E + e];
+        if constexpr (Seam) {
+            if (to < 0) {
+                const double2 fn = far_inward(side_far<Seam>(to), a.normal, a.link);
+                nx = R(fn.x);
+                ny = R(fn.y);
+            }
+        }
+        tr_out[side_far<Seam>(to) * n + (N - idx)] = characteristic(p, u, v, nx, ny);
     };
 
     if (active) {
@@ -705,8 +743,10 @@ __global__ void __launch_bounds__(256) line_trace_kernel(TraceArgs a, const __gr
         const int64_t e = (idx / (4 * n)) % K, inst = idx / (4 * n * K);
         const int2 lk = a.link[4 * e + s];
         if (((lk.y >> 2) & 7) != kInterior) continue;
-        const double2 nv = a.normal[4 * e + s];
-        const bool role = (lk.y >> 5) & 1;
+        const int64_t far = 4 * static_cast<int64_t>(lk.x) + (lk.y & 3);
+        double2 nv = a.normal[4 * e + s];
+        if ((lk.y >> 5) & 1) nv = double2{-nv.x, -nv.y};
+        if (lk.y & kSeamNormal) nv = far_inward(far, a.normal, a.link);
         const int line = (s < 2) ? m : N - m;
         const int base = (s == 0 || s == 2) ? line * n : line, stride = (s == 0 || s == 2) ? 1 : n;
         R t[3] = {0, 0, 0};
@@ -720,7 +760,7 @@ __global__ void __launch_bounds__(256) line_trace_kernel(TraceArgs a, const __gr
                 t[f] = fma((s == 0 || s == 3) ? cf.lm[j] : cf.lp[j], R(qe[j * stride]), t[f]);
             }
         }
-        out[((inst * Kp + lk.x) * 4 + (lk.y & 3)) * n + (N - m)] = characteristic(t[0], t[1], t[2], R(role ? -nv.x : nv.x), R(role ? -nv.y : nv.y));
+        out[(inst * Kp * 4 + far) * n + (N - m)] = characteristic(t[0], t[1], t[2], R(nv.x), R(nv.y));
     }
 }
 

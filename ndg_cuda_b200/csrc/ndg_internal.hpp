@@ -80,10 +80,12 @@ void init_adaptivity_state(Topology& topo);
 // Device plan of one mesh for the fused stage kernels (uniform order N,
 // conforming faces). Per domain element side:
 //   link.x = neighbour element whose side trace feeds the face (-1: none),
-//   link.y = neighbour side | kind << 2 | role << 5,
-// where kind is a SideKind and role is 1 when the element is the face's
-// right (second) element.
+//   link.y = neighbour side | kind << 2 | role << 5 | kSeamNormal,
+// where kind is a SideKind, role is 1 when the element is the face's right
+// (second) element, and kSeamNormal is set where the neighbour side's outward
+// normal is not the exact opposite of this side's (periodic seams).
 enum SideKind : int { kInterior = 0, kMirror = 1, kCopy = 2, kAnalytic = 3, kZero = 4 };
+constexpr int32_t kSeamNormal = 1 << 6;
 
 struct SidePlan {
     std::vector<int32_t> link;      // 2 per side, 8 per element

@@ -13,23 +13,23 @@ constexpr bool usable() {
 }
 
 template <int N, typename R>
-cudaError_t prepare() {
+cudaError_t prepare(bool seam) {
     if constexpr (usable<N, R>()) {
         constexpr int E = line_default_elements(N);
-        return cudaFuncSetAttribute(line_stage_kernel<N, R, E, SpeedStageArgs>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(LineTile<N, R, E>::kBytes));
+        return cudaFuncSetAttribute(seam ? line_stage_kernel<N, R, E, SpeedStageArgs, true> : line_stage_kernel<N, R, E, SpeedStageArgs, false>,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(LineTile<N, R, E>::kBytes));
     } else {
         return cudaErrorInvalidValue;
     }
 }
 
 template <int N, typename R>
-cudaError_t launch(const SpeedStageArgs& a, cudaStream_t stream) {
+cudaError_t launch(bool seam, const SpeedStageArgs& a, cudaStream_t stream) {
     if constexpr (usable<N, R>()) {
         constexpr int E = line_default_elements(N);
         using T = LineTile<N, R, E>;
-        return launch_dependent(line_stage_kernel<N, R, E, SpeedStageArgs>, dim3(static_cast<unsigned>((a.n_elements + E - 1) / E)), T::kThreads, T::kBytes,
-                                stream, a, make_line_coeffs<N, R>());
+        return launch_dependent(seam ? line_stage_kernel<N, R, E, SpeedStageArgs, true> : line_stage_kernel<N, R, E, SpeedStageArgs, false>,
+                                dim3(static_cast<unsigned>((a.n_elements + E - 1) / E)), T::kThreads, T::kBytes, stream, a, make_line_coeffs<N, R>());
     } else {
         return cudaErrorInvalidValue;
     }
@@ -54,9 +54,11 @@ cudaError_t launch(const SpeedStageArgs& a, cudaStream_t stream) {
         default: return cudaErrorInvalidValue;                                          \
     }
 
-cudaError_t prepare_speed_line(int N, bool fp32) { NDG_SPEED_LINE_DISPATCH(prepare) }
+cudaError_t prepare_speed_line(int N, bool fp32, bool seam) { NDG_SPEED_LINE_DISPATCH(prepare, seam) }
 
-cudaError_t launch_speed_line(int N, bool fp32, const SpeedStageArgs& a, cudaStream_t stream) { NDG_SPEED_LINE_DISPATCH(launch, a, stream) }
+cudaError_t launch_speed_line(int N, bool fp32, bool seam, const SpeedStageArgs& a, cudaStream_t stream) {
+    NDG_SPEED_LINE_DISPATCH(launch, seam, a, stream)
+}
 
 }  // namespace dev
 }  // namespace ndg

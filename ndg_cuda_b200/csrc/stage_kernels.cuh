@@ -77,11 +77,12 @@ int elements_per_block(int N);
 // one of them (FP64 default rounding, or the FP32 form).
 int tile_candidates_fp64(int N, bool line, int* out, int max);  // line: the line kernel's tiles
 int tile_candidates_fp32(int N, bool line, int* out, int max);
-cudaError_t prepare_stage_variant_fp64(int N, bool line, int epb);
-cudaError_t prepare_stage_variant_fp32(int N, bool line, int epb);
+cudaError_t prepare_stage_variant_fp64(int N, int epb);
+cudaError_t prepare_stage_variant_fp32(int N, int epb);
 cudaError_t launch_stage_variant_fp64(int N, int epb, const StageArgs& a, cudaStream_t stream);
 cudaError_t launch_stage_variant_fp32(int N, int epb, const StageArgs& a, cudaStream_t stream);
-// The line kernel (line_stage.cuh; elements = 0: its default tile): whether it
+// The line kernel (line_stage.cuh; elements = 0: its default tile; seam: of a
+// mesh with kSeamNormal sides, line_seam_*.cu): whether it
 // runs order N, its candidate tiles, and its first traces. Its traces are one
 // outgoing characteristic per side node, [instance][field_stride][side][N+1]
 // in the far slots, at the start of the trace buffers.
@@ -89,10 +90,14 @@ bool line_kernel_runs(int N, bool fp32, int64_t elements);  // elements of all i
 int line_default_tile(int N);
 int line_candidates_fp64(int N, int* out, int max);
 int line_candidates_fp32(int N, int* out, int max);
-cudaError_t prepare_line_fp64(int N, int elements);
-cudaError_t prepare_line_fp32(int N, int elements);
-cudaError_t launch_line_fp64(int N, int elements, const StageArgs& a, cudaStream_t stream);
-cudaError_t launch_line_fp32(int N, int elements, const StageArgs& a, cudaStream_t stream);
+cudaError_t prepare_line_fp64(int N, bool seam, int elements);
+cudaError_t prepare_line_fp32(int N, bool seam, int elements);
+cudaError_t launch_line_fp64(int N, bool seam, int elements, const StageArgs& a, cudaStream_t stream);
+cudaError_t launch_line_fp32(int N, bool seam, int elements, const StageArgs& a, cudaStream_t stream);
+cudaError_t prepare_line_seam_fp64(int N, int elements);
+cudaError_t prepare_line_seam_fp32(int N, int elements);
+cudaError_t launch_line_seam_fp64(int N, int elements, const StageArgs& a, cudaStream_t stream);
+cudaError_t launch_line_seam_fp32(int N, int elements, const StageArgs& a, cudaStream_t stream);
 cudaError_t launch_line_traces_fp64(int N, const TraceArgs& a, cudaStream_t stream);
 cudaError_t launch_line_traces_fp32(int N, const TraceArgs& a, cudaStream_t stream);
 // Tile codes at or above kTensorTile select the tensor-core contraction

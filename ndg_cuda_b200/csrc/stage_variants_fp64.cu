@@ -24,9 +24,8 @@ int tile_candidates_fp64(int N, bool line, int* out, int max) {
     return c + tile_candidates_tc64(N, out + c, max - c);
 }
 
-cudaError_t prepare_stage_variant_fp64(int N, bool line, int epb) {
+cudaError_t prepare_stage_variant_fp64(int N, int epb) {
     if (epb >= kTensorTile) return prepare_stage_variant_tc64(N, epb - kTensorTile);
-    if (line) return prepare_line_fp64(N, epb);
 #define NDG_CALL(n) return variant_prepare_n<false, n, false>(epb)
     NDG_VARIANT_ORDERS(NDG_CALL)
 #undef NDG_CALL

@@ -347,6 +347,14 @@ SidePlan build_side_plan(const Topology& t, const Tables& tables) {
             p.normal[2 * ps + 1] = t.face_normal[static_cast<size_t>(f)][1];
         }
     }
+    // Seams have two faces, each with a normal of its own.
+    for (size_t i = 0; i < static_cast<size_t>(4 * K); ++i) {
+        int32_t& word = p.link[2 * i + 1];
+        if (((word >> 2) & 7) != kInterior) continue;
+        const size_t o = 4 * static_cast<size_t>(p.link[2 * i]) + static_cast<size_t>(word & 3);
+        const double sign = ((word >> 5) & 1) == ((p.link[2 * o + 1] >> 5) & 1) ? -1.0 : 1.0;
+        if (p.normal[2 * i] != sign * p.normal[2 * o] || p.normal[2 * i + 1] != sign * p.normal[2 * o + 1]) word |= kSeamNormal;
+    }
     return p;
 }
 

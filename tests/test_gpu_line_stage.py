@@ -157,3 +157,51 @@ def test_fp32_speed_derivative_keeps_its_accuracy(N):
         return np.sqrt(err / size)
 
     assert rms(40) < 1.15 * rms(38)
+
+
+def _seam_zone(kind):
+    """Periodic squares whose seam sides are not exactly antiparallel: turned
+    by 0.3 rad (translates, normals equal to the rounding of the coordinates),
+    and bent into a ring's sector (the y seam's normals 0.5 rad apart)."""
+    zone = meshgen.uniform_zone(41, order="rowmajor", x_periodic=kind == "turned", y_periodic=True, boundary=meshgen.WALL, jitter=0.1, seed=4)
+    x, y = zone["x"].copy(), zone["y"].copy()
+    if kind == "turned":
+        zone["x"], zone["y"] = np.cos(0.3) * x - np.sin(0.3) * y, np.sin(0.3) * x + np.cos(0.3) * y
+    else:
+        zone["x"], zone["y"] = (3 + x) * np.cos(0.25 * y), (3 + x) * np.sin(0.25 * y)
+    return zone
+
+
+@pytest.mark.parametrize("precision", [ndg.FP64, ndg.FP32])
+@pytest.mark.parametrize("N", [3, 6, 8])
+@pytest.mark.parametrize("kind", ["turned", "sector"])
+def test_seams_whose_normals_are_not_opposite(N, kind, precision):
+    """The line kernel runs there too, and gives what the three-threads-a-line
+    kernel and the oracle give, forward, operator and transpose."""
+    zone = _seam_zone(kind)
+    o = OracleSolver(zone, N)
+    o.initial_conditions()
+    rng = np.random.default_rng(N)
+    m = ndg.Mesh2D_t(zone, N, precision=precision)
+    fields = [rng.standard_normal(m.field_size) for _ in range(3)]
+    assert m.stage_kernel().startswith("line_stage_kernel")
+    m.close()
+    line, = _run(zone, N, precision, False, fields, 1, 9)
+    three, = _run(zone, N, precision, True, fields, 1, 9)
+    assert rel_l2(line, three) < (1e-13 if precision == ndg.FP64 else 2e-6)
+    for f, v in zip(("p", "u", "v"), fields):
+        o.set_field(f, v)
+    o.run(9)
+    want = np.concatenate([o.field(f) for f in ("p", "u", "v")])
+    assert rel_l2(line[:want.size], want) < (1e-12 if precision == ndg.FP64 else 2e-6)
+    mesh = ndg.Mesh2D_t(zone, N)
+    c = 1.0 + 0.2 * rng.random(mesh.n_elements_)
+    adj = ndg.Adjoint2D_t(mesh, speed=c, precision=precision)
+    o.set_speed(c)
+    x, y = rng.standard_normal(3 * mesh.field_size), rng.standard_normal(3 * mesh.field_size)
+    Lx, LTy, dc = adj.operator(x, y)
+    LTy_o, dc_o = o.operator_transpose(x, y)
+    for got, ref in ((Lx, o.operator(x)), (LTy, LTy_o), (dc, dc_o)):
+        assert rel_l2(got, ref) < (1e-12 if precision == ndg.FP64 else 1e-6)
+    adj.close()
+    mesh.close()
