@@ -38,7 +38,7 @@ struct ndg_adjoint {
     bool fp32 = false;
     // The forward and adjoint stages run the line kernels in this form (by the
     // rule of the uniform stage), with one value per side node in tr and atr.
-    bool line() const { return ndg::dev::line_kernel_runs(N, fp32, K); }
+    bool line() const { return ctx->regular && ndg::dev::line_kernel_runs(N, fp32, K); }
     ndg::dev::Receivers rec{};
     // the last forward
     bool has_forward = false;

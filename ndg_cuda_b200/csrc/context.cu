@@ -203,11 +203,11 @@ cudaError_t issue_general_stage(ndg_ctx* c, int m, int in) {
 }
 
 // Whether the uniform stage of a form (FP64 default rounding, or FP32) runs the
-// line kernel (line_stage.cuh): on a mesh of its orders and sizes. The time
-// derivative (keep_derivative) is a by-product only of the three-threads-a-line
-// kernel.
+// line kernel (line_stage.cuh): on a mesh of its orders and sizes, without
+// degenerate elements (jacobians_regular). The time derivative
+// (keep_derivative) is a by-product only of the three-threads-a-line kernel.
 bool line_form(const ndg_ctx* c, bool f32) {
-    return !c->general && !c->keep_derivative && dev::line_kernel_runs(c->N, f32, c->K * c->n_instances);
+    return !c->general && c->regular && !c->keep_derivative && dev::line_kernel_runs(c->N, f32, c->K * c->n_instances);
 }
 
 // The kernel of the context's uniform stage: the one that runs a tile code
@@ -473,6 +473,7 @@ void upload_plan(ndg_ctx* c, const Layout& l) {
     if (!l.general) {
         if (c->N > kMaxOrder) fail(NDG_ERR_UNSUPPORTED, "orders above 16 have no compiled kernel");
         SidePlan plan = build_side_plan(c->topo, c->tables);
+        c->regular = jacobians_regular(plan, c->K, std::abs(c->tables.get(NDG_TABLE_NODES, c->N)[0]));
         c->seam_normals = false;
         for (size_t i = 0; i < 4 * K; ++i) c->seam_normals |= (plan.link[2 * i + 1] & kSeamNormal) != 0;
         // Tiles copy an even number of elements: pad the per-element arrays

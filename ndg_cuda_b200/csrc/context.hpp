@@ -113,6 +113,7 @@ struct ndg_ctx {
     bool traces_valid = false;
     bool line_traces = false;   // the traces hold the line kernel's characteristics
     bool seam_normals = false;  // the mesh has kSeamNormal sides
+    bool regular = true;        // jacobians_regular: the line kernels may run
     double dt_mesh = 0.0;
 
     // Mixed-order meshes (after adaptation) run the general stage path.

@@ -95,6 +95,10 @@ struct SidePlan {
     std::vector<double> corners;    // 8 per element: x0, y0, x1, y1, x2, y2, x3, y3
 };
 SidePlan build_side_plan(const Topology& topo, const Tables& tables);
+// Whether the Jacobian of every element is a normal number with a normal
+// reciprocal, and no difference of nearly equal terms, at all nodes of an order
+// whose outermost node is at distance t from the element's centre.
+bool jacobians_regular(const SidePlan& plan, int64_t K, double t);
 
 // True when every element and face has one order and every face is
 // conforming, so the fused uniform-order kernels apply.

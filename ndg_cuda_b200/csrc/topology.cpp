@@ -21,6 +21,7 @@
 #include <algorithm>
 #include <cmath>
 #include <fstream>
+#include <limits>
 #include <sstream>
 #include <unordered_map>
 
@@ -268,6 +269,31 @@ void compute_geometry(Topology& t, const Tables& tables) {
 // trace, outflow copies it scaled, inflow evaluates the analytic wave,
 // periodic ghosts copy the donor's trace, and a later list in that order
 // overrides an earlier one for the same ghost.
+bool jacobians_regular(const SidePlan& plan, int64_t K, double t) {
+    // x_xi and y_xi are linear in eta, x_eta and y_eta in xi, and so is J in each
+    // of them: between its values at the four outermost nodes, and its terms
+    // no larger than there.
+    for (int64_t e = 0; e < K; ++e) {
+        const double* c = plan.corners.data() + 8 * e;
+        double least = std::numeric_limits<double>::infinity(), most = 0.0, terms = 0.0;
+        int signs = 0;
+        for (int corner = 0; corner < 4; ++corner) {
+            const double xi = corner & 1 ? t : -t, eta = corner & 2 ? t : -t;
+            const double x_xi = 0.25 * ((1.0 - eta) * (c[2] - c[0]) + (1.0 + eta) * (c[4] - c[6]));
+            const double y_xi = 0.25 * ((1.0 - eta) * (c[3] - c[1]) + (1.0 + eta) * (c[5] - c[7]));
+            const double x_eta = 0.25 * ((1.0 - xi) * (c[6] - c[0]) + (1.0 + xi) * (c[4] - c[2]));
+            const double y_eta = 0.25 * ((1.0 - xi) * (c[7] - c[1]) + (1.0 + xi) * (c[5] - c[3]));
+            const double J = x_xi * y_eta - x_eta * y_xi, a = std::abs(J);
+            signs += J > 0.0 ? 1 : (J < 0.0 ? -1 : 0);
+            least = std::min(least, a);
+            most = std::max(most, a);
+            terms = std::max(terms, std::abs(x_xi * y_eta) + std::abs(x_eta * y_xi));
+        }
+        if (!(std::abs(signs) == 4 && least >= 0x1p-1000 && most <= 0x1p1000 && least >= 1e-12 * terms)) return false;
+    }
+    return true;
+}
+
 SidePlan build_side_plan(const Topology& t, const Tables& tables) {
     const int64_t K = t.n_domain;
     if (K <= 0) fail(NDG_ERR_MESH, "mesh has no domain elements");

@@ -205,3 +205,71 @@ def test_seams_whose_normals_are_not_opposite(N, kind, precision):
         assert rel_l2(got, ref) < (1e-12 if precision == ndg.FP64 else 1e-6)
     adj.close()
     mesh.close()
+
+
+def test_degenerate_elements_run_the_other_kernel():
+    """An element whose Jacobian vanishes at its nodes gives infinities in the
+    three-threads-a-line kernel, as an IEEE division does; the line kernel's
+    reciprocal has no special cases, so such a mesh does not run it. The same
+    mesh before its element collapses does, and so does one with a corner of an
+    element collapsed, whose nodes are regular."""
+    zone = meshgen.uniform_zone(41, order="rowmajor", boundary=meshgen.WALL)
+    quad = zone["sections"][0][4].reshape(-1, 4)[20 * 41 + 20] - 1
+
+    def kernel(points):
+        z = dict(zone, x=zone["x"].copy(), y=zone["y"].copy())
+        for node, (px, py) in points.items():
+            z["x"][quad[node]], z["y"][quad[node]] = px, py
+        out = []
+        for keep in (False, True):
+            m = ndg.Mesh2D_t(z, 6, keep_derivative=keep)
+            rng = np.random.default_rng(1)
+            for f in ("p", "u", "v"):
+                m.set_field(f, rng.standard_normal(m.field_size))
+            ndg.Solver2D_t.stage(m, 0, 0.0, 1e-3)
+            out.append(np.concatenate([m.get_field(f) for f in ("p", "u", "v", "k_p", "k_u", "k_v")]))
+            name = m.stage_kernel() if not keep else name
+            m.close()
+        return name, out[0], out[1]
+
+    name, line, three = kernel({})
+    assert name.startswith("line_stage_kernel") and rel_l2(line, three) < 1e-13
+    x, y = zone["x"][quad], zone["y"][quad]
+    name, line, three = kernel({2: (0.5 * (x[1] + x[3]), 0.5 * (y[1] + y[3]))})  # a triangle
+    assert name.startswith("line_stage_kernel") and rel_l2(line, three) < 1e-13
+    flat = {i: (0.25 * i, 0.0) for i in range(4)}  # four corners on a line
+    name, line, three = kernel(flat)
+    assert name.startswith("stage_kernel") and np.isinf(three).any()
+    assert np.array_equal(line, three, equal_nan=True)
+
+
+def test_line_reciprocal(tmp_path):
+    """line_rcp against the correctly rounded reciprocal, 6e7 arguments of both
+    signs: Jacobians of ordinary meshes (2^-60 to 2^60) and the whole range that
+    the kernels take (2^-1000 to 2^1000). Its error before the last rounding is
+    below 2^-79, so it may miss the correct rounding by one unit where 1 / x lies
+    that close to a boundary between two results: one random argument in 2^26,
+    and (2 - 2^-52) 2^k, whose reciprocal lies 2^-106 off one."""
+    import ctypes
+    import os
+    import subprocess
+
+    import torch
+    nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
+    if not os.path.exists(nvcc):
+        pytest.skip("no nvcc")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    out = str(tmp_path / "liblinercp.so")
+    subprocess.run([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC", "-shared",
+                    "-I", os.path.join(root, "include"), "-I", os.path.join(root, "ndg_cuda_b200", "csrc"),
+                    os.path.join(root, "tests", "cpp", "line_rcp.cu"), "-o", out], check=True, capture_output=True, text=True)
+    compare = ctypes.CDLL(out).compare_reciprocals
+    compare.argtypes = [ctypes.c_ulonglong, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_void_p]
+    torch.cuda.synchronize()
+    for low, high, near in ((-60, 60, 0), (-1000, 1000, 0), (-60, 60, 1), (-1000, 1000, 1)):
+        counts = torch.zeros(4, dtype=torch.int64, device="cuda")
+        torch.cuda.synchronize()
+        total = 592 * 256 * 400
+        assert compare(12345, low, high, near, 400, counts.data_ptr()) == 0
+        same, one, two, more = counts.tolist()
+        assert same + one == total and one <= (total / 15 if near else 20), (low, high, near, counts.tolist())
