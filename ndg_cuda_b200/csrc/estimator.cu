@@ -100,7 +100,8 @@ cudaError_t upload_polynomials(const Tables& t) {
         const auto& v = t.get(NDG_TABLE_POLYNOMIALS, N);
         std::copy(v.begin(), v.end(), poly.begin() + poly_offset(N));
     }
-    return cudaMemcpyToSymbol(c_poly, poly.data(), sizeof(double) * kPolyTotal);
+    // Only the orders of these tables: meshes of higher orders keep theirs.
+    return cudaMemcpyToSymbol(c_poly, poly.data(), sizeof(double) * static_cast<size_t>(poly_offset(std::min(t.N_max, kMaxPoly) + 1)));
 }
 
 cudaError_t launch_estimate_error(const EstimatorArgs& a, cudaStream_t stream) {

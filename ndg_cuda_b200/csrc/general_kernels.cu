@@ -1181,22 +1181,24 @@ cudaError_t upload_general_tables(const Tables& t) {
         const auto& d = t.get(NDG_TABLE_DERIVATIVE_MATRICES_HAT, N);
         std::copy(d.begin(), d.end(), dhat.begin() + gmat(N));
     }
+    // Only the orders of these tables: meshes of higher orders keep theirs.
+    const size_t vecs = static_cast<size_t>(gvec(std::min(t.N_max, kMaxOrder) + 1)), mats = static_cast<size_t>(gmat(std::min(t.N_max, kMaxOrder) + 1));
     cudaError_t err;
-    if ((err = cudaMemcpyToSymbol(g_nodes, nodes.data(), sizeof(double) * kGVecTotal)) != cudaSuccess) return err;
-    if ((err = cudaMemcpyToSymbol(g_weights, weights.data(), sizeof(double) * kGVecTotal)) != cudaSuccess) return err;
-    if ((err = cudaMemcpyToSymbol(g_inv_weights, inv_w.data(), sizeof(double) * kGVecTotal)) != cudaSuccess) return err;
-    if ((err = cudaMemcpyToSymbol(g_bary, bary.data(), sizeof(double) * kGVecTotal)) != cudaSuccess) return err;
-    if ((err = cudaMemcpyToSymbol(g_lagrange_left, ll.data(), sizeof(double) * kGVecTotal)) != cudaSuccess) return err;
-    if ((err = cudaMemcpyToSymbol(g_lagrange_right, lr.data(), sizeof(double) * kGVecTotal)) != cudaSuccess) return err;
-    if ((err = cudaMemcpyToSymbol(g_dhat, dhat.data(), sizeof(double) * kGMatTotal)) != cudaSuccess) return err;
+    if ((err = cudaMemcpyToSymbol(g_nodes, nodes.data(), sizeof(double) * vecs)) != cudaSuccess) return err;
+    if ((err = cudaMemcpyToSymbol(g_weights, weights.data(), sizeof(double) * vecs)) != cudaSuccess) return err;
+    if ((err = cudaMemcpyToSymbol(g_inv_weights, inv_w.data(), sizeof(double) * vecs)) != cudaSuccess) return err;
+    if ((err = cudaMemcpyToSymbol(g_bary, bary.data(), sizeof(double) * vecs)) != cudaSuccess) return err;
+    if ((err = cudaMemcpyToSymbol(g_lagrange_left, ll.data(), sizeof(double) * vecs)) != cudaSuccess) return err;
+    if ((err = cudaMemcpyToSymbol(g_lagrange_right, lr.data(), sizeof(double) * vecs)) != cudaSuccess) return err;
+    if ((err = cudaMemcpyToSymbol(g_dhat, dhat.data(), sizeof(double) * mats)) != cudaSuccess) return err;
     auto to_f = [](const std::vector<double>& v) { return std::vector<float>(v.begin(), v.end()); };
     const std::vector<float> fn = to_f(nodes), fw = to_f(weights), fiw = to_f(inv_w), fll = to_f(ll), flr = to_f(lr), fd = to_f(dhat);
-    if ((err = cudaMemcpyToSymbol(gf_nodes, fn.data(), sizeof(float) * kGVecTotal)) != cudaSuccess) return err;
-    if ((err = cudaMemcpyToSymbol(gf_weights, fw.data(), sizeof(float) * kGVecTotal)) != cudaSuccess) return err;
-    if ((err = cudaMemcpyToSymbol(gf_inv_weights, fiw.data(), sizeof(float) * kGVecTotal)) != cudaSuccess) return err;
-    if ((err = cudaMemcpyToSymbol(gf_lagrange_left, fll.data(), sizeof(float) * kGVecTotal)) != cudaSuccess) return err;
-    if ((err = cudaMemcpyToSymbol(gf_lagrange_right, flr.data(), sizeof(float) * kGVecTotal)) != cudaSuccess) return err;
-    return cudaMemcpyToSymbol(gf_dhat, fd.data(), sizeof(float) * kGMatTotal);
+    if ((err = cudaMemcpyToSymbol(gf_nodes, fn.data(), sizeof(float) * vecs)) != cudaSuccess) return err;
+    if ((err = cudaMemcpyToSymbol(gf_weights, fw.data(), sizeof(float) * vecs)) != cudaSuccess) return err;
+    if ((err = cudaMemcpyToSymbol(gf_inv_weights, fiw.data(), sizeof(float) * vecs)) != cudaSuccess) return err;
+    if ((err = cudaMemcpyToSymbol(gf_lagrange_left, fll.data(), sizeof(float) * vecs)) != cudaSuccess) return err;
+    if ((err = cudaMemcpyToSymbol(gf_lagrange_right, flr.data(), sizeof(float) * vecs)) != cudaSuccess) return err;
+    return cudaMemcpyToSymbol(gf_dhat, fd.data(), sizeof(float) * mats);
 }
 
 cudaError_t prepare_general_kernels(int N, int side_slots) {

@@ -52,6 +52,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 namespace ndg {
@@ -205,9 +206,13 @@ __global__ void set_step_kernel(double* step, double time, double dt, double dt_
 }
 
 // ---------------------------------------------------------------------------
-// Host copies of the packed tables (set by upload_tables): the stage kernels
-// take their order's coefficients as a by-value parameter.
+// Host copies of the packed tables (upload_tables adds the orders it brings; an
+// order's values never change): the stage kernels take their order's
+// coefficients as a by-value parameter, formed at every launch or capture, also
+// after another context has loaded a mesh of lower orders.
 namespace {
+std::mutex h_mutex;
+int h_N_max = -1;
 std::vector<double> h_nodes(kVecTotal), h_weights(kVecTotal), h_inv_weights(kVecTotal), h_ll(kVecTotal), h_lr(kVecTotal), h_dhat(kMatTotal);
 }
 
@@ -472,19 +477,28 @@ cudaError_t upload_tables(const Tables& t) {
         }
         for (int i = 0; i < n * n; ++i) dhat[static_cast<size_t>(mat_offset(N) + i)] = t.get(NDG_TABLE_DERIVATIVE_MATRICES_HAT, N)[static_cast<size_t>(i)];
     }
-    h_nodes = nodes;
-    h_weights = weights;
-    h_inv_weights = inv_w;
-    h_ll = ll;
-    h_lr = lr;
-    h_dhat = dhat;
+    const int N_max = std::min(t.N_max, kMaxOrder);
+    const size_t vecs = static_cast<size_t>(vec_offset(N_max + 1)), mats = static_cast<size_t>(mat_offset(N_max + 1));
+    {
+        std::lock_guard<std::mutex> lock(h_mutex);
+        if (N_max > h_N_max) {
+            const size_t v = static_cast<size_t>(vec_offset(h_N_max + 1)), m = static_cast<size_t>(mat_offset(h_N_max + 1));
+            std::copy(nodes.begin() + v, nodes.begin() + vecs, h_nodes.begin() + v);
+            std::copy(weights.begin() + v, weights.begin() + vecs, h_weights.begin() + v);
+            std::copy(inv_w.begin() + v, inv_w.begin() + vecs, h_inv_weights.begin() + v);
+            std::copy(ll.begin() + v, ll.begin() + vecs, h_ll.begin() + v);
+            std::copy(lr.begin() + v, lr.begin() + vecs, h_lr.begin() + v);
+            std::copy(dhat.begin() + m, dhat.begin() + mats, h_dhat.begin() + m);
+            h_N_max = N_max;
+        }
+    }
     cudaError_t err;
-    if ((err = cudaMemcpyToSymbol(c_nodes, nodes.data(), sizeof(double) * kVecTotal)) != cudaSuccess) return err;
-    if ((err = cudaMemcpyToSymbol(c_weights, weights.data(), sizeof(double) * kVecTotal)) != cudaSuccess) return err;
-    if ((err = cudaMemcpyToSymbol(c_inv_weights, inv_w.data(), sizeof(double) * kVecTotal)) != cudaSuccess) return err;
-    if ((err = cudaMemcpyToSymbol(c_lagrange_left, ll.data(), sizeof(double) * kVecTotal)) != cudaSuccess) return err;
-    if ((err = cudaMemcpyToSymbol(c_lagrange_right, lr.data(), sizeof(double) * kVecTotal)) != cudaSuccess) return err;
-    return cudaMemcpyToSymbol(c_dhat, dhat.data(), sizeof(double) * kMatTotal);
+    if ((err = cudaMemcpyToSymbol(c_nodes, nodes.data(), sizeof(double) * vecs)) != cudaSuccess) return err;
+    if ((err = cudaMemcpyToSymbol(c_weights, weights.data(), sizeof(double) * vecs)) != cudaSuccess) return err;
+    if ((err = cudaMemcpyToSymbol(c_inv_weights, inv_w.data(), sizeof(double) * vecs)) != cudaSuccess) return err;
+    if ((err = cudaMemcpyToSymbol(c_lagrange_left, ll.data(), sizeof(double) * vecs)) != cudaSuccess) return err;
+    if ((err = cudaMemcpyToSymbol(c_lagrange_right, lr.data(), sizeof(double) * vecs)) != cudaSuccess) return err;
+    return cudaMemcpyToSymbol(c_dhat, dhat.data(), sizeof(double) * mats);
 }
 
 }  // namespace dev

@@ -193,3 +193,49 @@ def test_tiles_are_those_of_the_kernel_that_runs(N, res, precision):
     tile, ms = mesh.autotune(3)
     assert ms > 0 and (tile == 0 or tile in mesh.tile_candidates()[0])
     mesh.close()
+
+
+@pytest.mark.parametrize("kind", ["uniform", "uniform fp32", "mixed", "mixed fp32", "adjoint"])
+def test_a_mesh_of_lower_order_loaded_meanwhile_changes_nothing(kind):
+    """Kernels take their order's coefficients from tables that every context
+    shares; another context's mesh of lower orders must not take them away,
+    from launches, captures of a later run, estimates or the adjoint."""
+    zone = meshgen.uniform_zone(8, boundary=meshgen.WALL)
+    precision = ndg.FP32 if "fp32" in kind else ndg.FP64
+
+    def low():
+        m = ndg.Mesh2D_t(zone, 2)
+        m.initial_conditions()
+        ndg.Solver2D_t.run(m, 1)
+        m.synchronize()
+        m.close()
+
+    results = []
+    for between in (lambda: None, low):
+        m = ndg.Mesh2D_t(zone, 5, maximum_N=9, precision=precision, tolerance_min=1e-12)
+        m.initial_conditions()
+        if kind == "adjoint":
+            adj = ndg.Adjoint2D_t(m, [[0.3, 0.2]])
+            p0 = m.get_field("p")
+            dt = adj.delta_t(0.5)
+            out = []
+            for _ in range(2):
+                between()
+                out += [adj.forward(p0, dt, 3, targets=np.zeros((4, 1)))[1].ravel(), adj.backward()["c"]]
+            adj.close()
+        else:
+            if "mixed" in kind:
+                between()
+                m.adapt((np.arange(64) % 2).astype(np.int32), np.full(64, 2.0))
+            t = ndg.Solver2D_t.run(m, 8)
+            between()
+            t = ndg.Solver2D_t.run(m, 1, t)  # a run that captures anew
+            between()
+            ndg.Solver2D_t.stage(m, 1, t, 1e-3)
+            between()
+            m.estimate_error()
+            out = [m.get_field(f) for f in ("p", "u", "v", "k_p")] + [m.error()[k] for k in ("p_error", "p_sigma")]
+        m.close()
+        results.append(np.concatenate(out))
+    assert np.isfinite(results[0]).all() and np.linalg.norm(results[0]) > 0
+    assert np.array_equal(results[0], results[1])
