@@ -42,6 +42,7 @@
 
 #include <algorithm>
 #include <cfloat>
+#include <mutex>
 #include <vector>
 
 namespace ndg {
@@ -1109,18 +1110,31 @@ cudaError_t launch_queue_t(const GeneralStage& a, const StageQueue& wq, cudaStre
     return cudaGetLastError();
 }
 
+// Lets a kernel be launched with `bytes` of dynamic shared memory. The limit is
+// the function's, for all contexts, and the tiles' sizes depend on the mesh
+// (side_slots), so it only rises.
+template <typename K>
+cudaError_t raise_shared(K* kernel, int bytes) {
+    static std::mutex mutex;
+    std::lock_guard<std::mutex> lock(mutex);
+    cudaFuncAttributes attr{};
+    const cudaError_t err = cudaFuncGetAttributes(&attr, kernel);
+    if (err != cudaSuccess || attr.maxDynamicSharedSizeBytes >= bytes) return err;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+}
+
 template <int N>
 cudaError_t set_attrs(int side_slots) {
     const int b64 = static_cast<int>(FusedTile<N, double>::bytes(side_slots));
     const int b32 = static_cast<int>(FusedTile<N, float>::bytes(side_slots));
-    cudaError_t err = cudaFuncSetAttribute(general_fused_kernel<N, false, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, b64);
-    if (err == cudaSuccess) err = cudaFuncSetAttribute(general_fused_kernel<N, true, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, b64);
-    if (err == cudaSuccess) err = cudaFuncSetAttribute(general_fused_kernel<N, false, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, b32);
+    cudaError_t err = raise_shared(general_fused_kernel<N, false, double>, b64);
+    if (err == cudaSuccess) err = raise_shared(general_fused_kernel<N, true, double>, b64);
+    if (err == cudaSuccess) err = raise_shared(general_fused_kernel<N, false, float>, b32);
     const int f64 = static_cast<int>(FluxTile<N, double>::bytes(side_slots));
     const int f32 = static_cast<int>(FluxTile<N, float>::bytes(side_slots));
-    if (err == cudaSuccess) err = cudaFuncSetAttribute(side_flux_kernel<N, false, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, f64);
-    if (err == cudaSuccess) err = cudaFuncSetAttribute(side_flux_kernel<N, true, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, f64);
-    if (err == cudaSuccess) err = cudaFuncSetAttribute(side_flux_kernel<N, false, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, f32);
+    if (err == cudaSuccess) err = raise_shared(side_flux_kernel<N, false, double>, f64);
+    if (err == cudaSuccess) err = raise_shared(side_flux_kernel<N, true, double>, f64);
+    if (err == cudaSuccess) err = raise_shared(side_flux_kernel<N, false, float>, f32);
     return err;
 }
 
@@ -1270,9 +1284,9 @@ int general_tile_elements(int N) {
 
 cudaError_t prepare_general_queue(size_t smem_bytes) {
     const int b = static_cast<int>(smem_bytes);
-    cudaError_t err = cudaFuncSetAttribute(general_stage_kernel<false, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    if (err == cudaSuccess) err = cudaFuncSetAttribute(general_stage_kernel<true, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    if (err == cudaSuccess) err = cudaFuncSetAttribute(general_stage_kernel<false, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+    cudaError_t err = raise_shared(general_stage_kernel<false, double>, b);
+    if (err == cudaSuccess) err = raise_shared(general_stage_kernel<true, double>, b);
+    if (err == cudaSuccess) err = raise_shared(general_stage_kernel<false, float>, b);
     return err;
 }
 

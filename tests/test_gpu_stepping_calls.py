@@ -239,3 +239,35 @@ def test_a_mesh_of_lower_order_loaded_meanwhile_changes_nothing(kind):
         results.append(np.concatenate(out))
     assert np.isfinite(results[0]).all() and np.linalg.norm(results[0]) > 0
     assert np.array_equal(results[0], results[1])
+
+
+@pytest.mark.parametrize("precision", [ndg.FP64, ndg.FP32])
+@pytest.mark.parametrize("mode", [0, 1, 2])
+def test_a_mixed_mesh_with_smaller_tiles_loaded_meanwhile_changes_nothing(mode, precision):
+    """Split meshes need larger mixed-order tiles than p-adapted ones of the
+    same orders; the kernels' shared-memory limit is one for all contexts."""
+    zone = meshgen.uniform_zone(8, boundary=meshgen.WALL)
+
+    def mixed(split):
+        m = ndg.Mesh2D_t(zone, 8, maximum_N=12, max_split_level=2 if split else 0, precision=precision)
+        m.set_mixed_launch(mode)
+        m.initial_conditions()
+        for _ in range(2):
+            K = m.n_elements_
+            m.adapt((np.arange(K) % 3 == 0).astype(np.int32), np.where(np.arange(K) % 2 == 0, 0.5, 2.0) if split else np.full(K, 2.0))
+        return m
+
+    results = []
+    for between in (False, True):
+        m = mixed(True)
+        t = ndg.Solver2D_t.run(m, 1)
+        if between:
+            other = mixed(False)
+            ndg.Solver2D_t.run(other, 1)
+            other.synchronize()
+            other.close()
+        t = ndg.Solver2D_t.run(m, 2, t)  # captures the graph of the other parity
+        ndg.Solver2D_t.stage(m, 1, t, 1e-4)
+        results.append(_get(m))
+        m.close()
+    assert np.isfinite(results[0]).all() and np.array_equal(results[0], results[1])
