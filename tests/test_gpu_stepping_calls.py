@@ -127,7 +127,7 @@ def _launched(mesh, steps=1):
     from torch.profiler import ProfilerActivity, profile
     ndg.Solver2D_t.run(mesh, steps)
     mesh.synchronize()
-    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+    with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as prof:
         ndg.Solver2D_t.run(mesh, steps)
         mesh.synchronize()
     names = [e.name for e in prof.events() if "stage_kernel" in e.name]
