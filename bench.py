@@ -154,11 +154,11 @@ def measured_hbm_peak() -> tuple[float, str]:
         return 6650.0, "fallback"
 
 
-def profiled_traffic(tile: int = 0) -> float | None:
-    """DRAM bytes per stage-kernel launch of the tile in use (0: the default)
-    from the committed ncu summary."""
+def profiled_traffic(kernel: str) -> float | None:
+    """DRAM bytes per launch of a stage kernel on the benchmark's mesh from the
+    committed ncu summary (None where it has no capture of that kernel)."""
     path = os.path.join(ROOT, "profiles", "stage_kernel_traffic.txt")
-    key = f"N{ORDER}_res{RES}" + (f"_tile{tile}" if tile else "")
+    key = f"{kernel.replace(' ', '')}_res{RES}"
     try:
         with open(path) as f:
             for line in f:
@@ -405,7 +405,7 @@ def order_sweep_leg(local: int, stream) -> dict:
                           "dof": dof, "value": dof * 3 * SWEEP_STEPS / wall, "unit": "DOF-stage updates/s",
                           "reference_a100_ms": SWEEP_A100_MS[N], "speedup_vs_reference_a100": SWEEP_A100_MS[N] / ms,
                           "reference_cpu_core_ms": SWEEP_CPU_CORE_MS[N], "elements_after": m.n_elements_,
-                          "tile_elements_per_cta": tile or "default"}
+                          "tile_elements_per_cta": tile or m.tile_candidates()[1]}
         m.close()
     return {"workload": f"dg_wave_rk3_inflow_{SWEEP_RES}x{SWEEP_RES}_unit_square_plane_wave_N4to16",
             "setup": (f"{SWEEP_RES}x{SWEEP_RES} quads on [0,1]^2, boundaries held to the analytic plane wave, CFL {CFL}, FP64, "
@@ -445,7 +445,7 @@ def published_runs_leg(local: int, stream) -> dict:
                      "wall_s": wall, "device_s": e0.elapsed_time(e1) / 1e3, "value": dof * 3 * steps / wall,
                      "unit": "DOF-stage updates/s", "reference_wall_s": ref_s, "reference_hardware": hardware,
                      "speedup_vs_reference": ref_s / wall, "l2_vs_analytic": dict(zip("puv", map(float, m.l2_error(t)))),
-                     "tile_elements_per_cta": tile or "default"})
+                     "tile_elements_per_cta": tile or m.tile_candidates()[1]})
         m.close()
     return {"setup": f"unit square, boundaries held to the analytic plane wave, CFL {CFL}, FP64, t = 0 to 2 s, no adaptivity",
             "reference_numbers": "published wall times of the reference (thesis plots.py:22, 101-104)", "runs": runs}
@@ -606,7 +606,7 @@ def batched_leg(local: int, stream, peak: float, dist) -> dict:
         out[name] = {"value": world * dof * 3 * BATCH_STEPS / (ms / 1e3), "unit": "DOF-stage updates/s", "ms_per_step": ms / BATCH_STEPS,
                      "kernel_ms": stage_ms, "roofline_frac": BYTES_PER_DOF_STAGE * dof / (stage_ms / 1e3) / 1e9 / peak,
                      "per_stage": st["per_stage"], "kernel_ms_per_step": st["sum_ms"],
-                     "tile": {"elements_per_cta": tile if tile else "default", "autotuner_choice": "candidate" if tile else "default",
+                     "tile": {"elements_per_cta": tile if tile else m.tile_candidates()[1], "autotuner_choice": "candidate" if tile else "default",
                               "candidates": m.tile_candidates()[0], "tuned_ms_per_launch": tile_ms}}
         out["dof"] = dof
     # FP32 against FP64 after the configuration's steps from the same state
@@ -781,7 +781,8 @@ def run_ours(args) -> None:
     stage_ms = stages["mean_ms"]
     achieved = BYTES_PER_DOF_STAGE * dof / (stage_ms / 1e3) / 1e9
     peak, peak_kind = measured_hbm_peak()
-    traffic = profiled_traffic(tile)
+    kernel = mesh.stage_kernel()
+    traffic = profiled_traffic(kernel)
 
     # End to end through the C ABI with pinned host buffers.
     e2e_steps = 0 if args.no_e2e else 2
@@ -846,10 +847,10 @@ def run_ours(args) -> None:
             a64, a32 = mesh.get_field(f), m32.get_field(f)
             err[f] = float(((a32 - a64) ** 2).sum() ** 0.5 / max((a64 ** 2).sum() ** 0.5, 1e-300))
         fp32 = {"value": world * dof * 3 * args.steps / (float(f_ms.item()) / 1e3), "unit": "DOF-stage updates/s",
-                "ms_per_step": float(f_ms.item()) / args.steps, "kernel": f"stage_kernel_f32<{ORDER}>", "kernel_ms": stage32_ms,
+                "ms_per_step": float(f_ms.item()) / args.steps, "kernel": m32.stage_kernel(), "kernel_ms": stage32_ms,
                 "per_stage": st32["per_stage"], "kernel_ms_per_step": st32["sum_ms"],
                 "roofline_frac": BYTES_PER_DOF_STAGE * dof / (stage32_ms / 1e3) / 1e9 / peak,
-                "rel_l2_vs_fp64": err, "steps_compared": CONFIG_STEPS, "tile_elements_per_cta": tile32 or "default",
+                "rel_l2_vs_fp64": err, "steps_compared": CONFIG_STEPS, "tile_elements_per_cta": tile32 or m32.tile_candidates()[1],
                 "l2_vs_analytic": l2_analytic,
                 "wall_time_per_unit_time_s": float(f_ms.item()) / args.steps / 1e3 / dt_step,
                 "arithmetic": "traces, fluxes, metrics and volume term in FP32; q, k and the RK update in FP64"}
@@ -889,10 +890,10 @@ def run_ours(args) -> None:
                         "d2h_bytes_per_step": state_bytes, "rk3_steps_per_e2e_step": CONFIG_STEPS, "e2e_steps": e2e_steps,
                         "host_wall_s": wall},
                 "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                             "traffic": traffic, "kernel": f"line_stage_kernel<{ORDER}, double, {tile or 16}>" if tile < 100 else f"stage_kernel<{ORDER}, false, {tile - 100}, true>", "kernel_ms": stage_ms,
+                             "traffic": traffic, "kernel": kernel, "kernel_ms": stage_ms,
                              "per_stage": stages["per_stage"], "kernel_ms_per_step": stages["sum_ms"],
                              "ms_per_step_device": ms_max / args.steps,
-                             "tile_elements_per_cta": tile or "default",
+                             "tile_elements_per_cta": tile or mesh.tile_candidates()[1],
                              "tile_source": "autotuner" if args.tile is None else "--tile",
                              "algorithmic_bytes_per_launch": BYTES_PER_DOF_STAGE * dof, "peak_source": peak_kind},
                 "cpu_baseline": None if cpu is None else {k: cpu[k] for k in ("value", "unit", "cores", "kind", "sample")},
