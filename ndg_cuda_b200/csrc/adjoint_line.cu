@@ -16,11 +16,18 @@
 // receiving element applies the sender's normal: the opposite of its own, or on
 // a seam (kSeamNormal) the neighbour side's.
 //
-// Measured, backward of 60 steps with checkpoints every 20 at 96 x 96 (its
-// recomputation included), ms, against three threads a line: FP64 N = 4 2.00
-// (4.65), N = 6 3.52 (6.86), N = 7 5.07 (7.76), N = 8 5.89 (10.39), N = 9 10.03
-// (13.68); FP32 form N = 4 2.15 (3.41), N = 6 3.98 (6.23), N = 8 6.21 (9.10).
-// Nine field tiles an element bound the tiles per SM; latency is what is left.
+// Measured, backward of 60 steps with checkpoints every 20 (its recomputation
+// included), ms, in parentheses three threads a line with the same launches. At
+// 96 x 96, FP64: N = 1 1.18 (3.07), 2 1.39 (3.67), 3 1.80 (3.60), 4 1.97 (4.85), 5
+// 2.91 (6.51), 6 3.54 (7.88), 7 5.09 (8.10), 8 5.89 (11.7), 9 10.1 (14.3), 10 10.7
+// (18.9), 11 16.1 (22.8), 12 19.8 (26.8); FP32 form: N = 1 1.20 (2.29), 2 1.34
+// (2.79), 3 1.96 (2.82), 4 2.13 (3.58), 5 3.03 (5.42), 6 3.90 (6.68), 8 6.14
+// (9.62), 10 12.2 (16.1). By the size rule of the forward (kLineMinElements): at
+// 1,600 elements FP64 N = 5 1.41 (1.97), 8 1.93 (2.77), 12 3.41 (6.14), FP32 N = 8
+// 2.18 (2.74); at 100 elements N = 1 1.15 (1.37), 4 1.09 (1.58). The forward of
+// the same steps is ahead too but for N = 9 and FP32 N = 10 below 2,304 elements
+// (1.79 against 1.70, 1.71 against 1.57). Nine field tiles an element bound the
+// tiles per SM (N = 7: 2, 7.5 warps); latency is what is left.
 #include "adjoint.cuh"
 #include "line_stage.cuh"
 
@@ -409,9 +416,11 @@ __global__ void __launch_bounds__(AdjLineTile<N, R, E>::kThreads, AdjLineTile<N,
 }
 
 // Elements a tile, by the measure above (96 x 96, ms, with 16 / 8 / 4): FP64 N =
-// 4 2.00 / 2.45 / 2.61, N = 6 3.52 / 4.29 / 4.24, N = 7 5.07 / 5.46 / 5.53, N =
-// 8 5.89 / 7.31 / 8.78, N = 9 10.71 / 10.03 / 10.19; above order 10 a tile of 8
-// is alone on its SM.
+// 1 1.26 / 1.25 / 1.55, 2 1.45 / 1.54 / 1.65, 3 1.84 / 1.90 / 2.05, 4 2.01 / 2.44
+// / 2.59, 5 2.89 / 3.47 / 3.66, 6 3.53 / 4.34 / 4.24, 7 5.09 / 5.46 / 5.51, 8 5.87
+// / 7.33 / 8.78, 9 10.71 / 10.13 / 10.16, 10 10.78 / 12.09 / 12.16, 11 (8 / 4)
+// 16.23 / 16.18, 12 19.50 / 19.84; FP32 N = 5 2.94 / 3.14 / 3.83, 8 6.10 / 7.38 /
+// 8.03, 10 12.21 / 12.94 / 12.85.
 template <int N>
 constexpr int elements() {
     return N <= 8 || N == 10 ? 16 : (N <= 10 ? 8 : 4);

@@ -8,7 +8,7 @@
 //    the contraction serves three fields. A stage takes two passes over
 //    shared memory: columns (xi: k <- a k + G_xi), then rows (eta: k <- k +
 //    G_eta, q <- q + g dt k), then the column traces of the new q. N = 8,
-//    256 x 256, FP64: 44.5 M warp instructions instead of 94.7 M and 12.7 M
+//    256 x 256, FP64: 39.1 M warp instructions instead of 94.7 M and 13.8 M
 //    shared wavefronts instead of 25.5 M per launch.
 //  - The face flux reads the far side only through its outgoing
 //    characteristic w = p - (u, v) . n (n this side's outward normal), so sides
@@ -27,16 +27,20 @@
 // padding per element is needed, which rules the bulk copies out. Tiles of
 // fewer elements take bank::search's strides.
 //
-// Measured, us per launch (second and third stages; FP64 / FP32 form),
-// against the three-threads-a-line kernel with its best tile:
-//   N = 2, 256^2:  18.9 /  16.9 (49.6 /  45.6)   N = 8,  256^2:  97.7 / 100.8 (149.8 / 129.4)
-//   N = 4, 256^2:  34.8 /  33.0 (63.8 /  56.4)   N = 10, 192^2:  86.1 /  96.2 (131.4 / 113.9)
-//   N = 5, 256^2:  57.8 /  57.8 (92.7 /  84.3)   N = 12, 160^2: 111.8 / 120.2 (123.3 / 104.8)
-//   N = 6, 256^2:  63.7 /  62.5 (104.8 / 91.0)   N = 16, 128^2: 167.8 / 128.4 (139.8 / 121.5)
-//   N = 7, 256^2:  94.6 / 100.4 (122.5 / 98.0)
-// N = 8 moves about 560 MB a launch, 84 us at the 6650 GB/s copy rate; what
-// is left is latency: 3 tiles (15 warps) an SM, held there by shared memory
-// (q and k) and registers.
+// Measured, us per launch by events (second and third stages, the best tile of
+// each kernel; FP64 / FP32 form), in parentheses the three-threads-a-line
+// kernel:
+//   N = 2, 256^2:  18.9 /  16.8 (45.3 / 45.4)     N = 8,  256^2: 101.4 / 102.0 (151.1 / 130.2)
+//   N = 4, 256^2:  36.3 /  33.9 (63.9 / 57.3)     N = 9,  192^2:  96.5 / 106.7 (117.1 /  97.6)
+//   N = 5, 256^2:  59.7 /  59.9 (93.2 / 84.3)     N = 10, 192^2:  93.6 /  95.6 (131.5 / 115.0)
+//   N = 6, 256^2:  65.1 /  63.6 (104.9 / 92.4)    N = 11, 192^2: 129.8 / 156.7 (156.1 / 133.5)
+//   N = 7, 256^2:  94.6 / 108.7 (123.3 / 98.6)    N = 12, 160^2: 116.2 / 126.2 (124.6 / 106.8)
+// In a run the launches overlap: N = 8 94.0 / 97.6 us a stage, N = 7 89.6, N = 5
+// 52.3 / 52.7, N = 2 14.1 / 12.0. N = 8 moves 502 MB a launch (part of its traces
+// stays in L2), 77 us at the 6541 GB/s copy rate; what is left is latency: 3 tiles
+// (15 warps) an SM, held there by shared memory (q and k) and registers alike.
+// Figures below that compare variants of the kernel are theirs, from before the
+// launches overlapped.
 #pragma once
 
 #include "adjoint.cuh"
@@ -57,24 +61,30 @@ namespace dev {
 // FP64 up to N = 14: from N = 15 a line's registers (3 (N + 1) values and
 // the accumulators) and the tile leave 6 warps an SM and it loses (N = 15
 // even, N = 16 167.8 against 139.8 us). FP32 form: q and k stay FP64 in
-// shared memory, so it pays only where the tile is contiguous or small: it
-// gains for N <= 6, N = 8 and N = 10, and loses 2% at N = 7 and 9 and 14% at
-// N = 12.
+// shared memory, so it pays only where the tile is contiguous or small: N <= 6,
+// N = 8 and N = 10. At N = 7 (256^2) and 9 (192^2) a run takes 95.9 against 92.7
+// and 101.4 against 93.1 us a stage, at N = 11 and 12 142 against 127 and 129
+// against 99.
 constexpr bool line_order(int N, bool fp32) { return fp32 ? (N <= 6 || N == 8 || N == 10) : N <= 14; }
 // On a mesh whose tiles all run at once a stage takes one thread's chain of
 // passes, a third as long with three threads a line. Up to N = 4 the line
-// kernel is even or ahead at every size; above, from kLineMinElements
-// elements (times the instances). us per stage of a run, line / three threads
-// a line, at 1,024 and 2,304 elements: FP64 N = 6 6.3 / 6.3 and 6.3 / 7.2 (at
-// 256 6.3 / 6.0), N = 8 7.7 / 7.0 and 7.7 / 8.4, N = 10 8.5 / 8.3 and 9.7 /
-// 11.1, N = 14 11.1 / 10.4 and 13.8 / 18.0; FP32 form N = 6 6.6 / 6.7 and 6.6
-// / 7.3, N = 8 7.7 / 7.0 and 8.3 / 8.4.
+// kernel is ahead or within 4% at every size (64 elements: N = 1 3.1 / 4.3, N = 3
+// 3.3 / 3.3, N = 4 3.6 / 3.7, FP32 N = 4 3.9 / 4.2 us per stage of a run, line /
+// three threads a line); above, from kLineMinElements elements (times the
+// instances). us per stage of a run at 1,024, 1,600 and 2,304 elements: FP64 N =
+// 5 4.6 / 4.4, 4.7 / 5.1 and 5.0 / 5.5, N = 6 4.7 / 4.9, 4.9 / 5.5 and 5.3 / 6.0,
+// N = 8 6.1 / 5.3, 6.2 / 6.2 and 6.8 / 7.4, N = 10 7.4 / 7.0, 7.4 / 8.5 and 8.0 /
+// 10.2, N = 14 10.6 / 9.1, 12.0 / 11.7 and 12.5 / 15.9; FP32 N = 6 5.1 / 5.1, 5.3
+// / 5.5 and 5.9 / 5.9, N = 10 7.9 / 6.8, 7.9 / 7.6 and 8.3 / 9.0. Two orders cross
+// later than the rule, at about 4,096: FP64 N = 7 (5.7 / 4.9, 6.5 / 5.5 and 7.1 /
+// 6.3; 4,096 8.8 / 8.7) and FP32 N = 8 (6.5 / 5.4, 6.6 / 6.0 and 7.7 / 6.8; 4,096
+// 9.8 / 9.1).
 constexpr bool line_every_size(int N) { return N <= 4; }
 constexpr int64_t kLineMinElements = 1536;
-// 16 elements up to N = 10 (8 within 3% at N = 7 and 9, slower elsewhere: N =
-// 8 122.9 against 97.7 us; 32 slower: 145). Above, a tile of 16 is alone on
-// its SM: 8 for odd N + 1 (N = 12: 111.8 us, 4: 127.0, 16: 117.2), 4 for even
-// (N = 11: 104.9, 8: 119.1, 16: 153.8).
+// 16 elements up to N = 10 (8 as fast at N = 9, 4% faster at N = 7 with a launch
+// on its own, 94.6 us against 98.6; slower elsewhere: N = 8 130.4 against 101.4;
+// 32 slower: 145). Above, a tile of 16 is alone on its SM: 8 for even N (N =
+// 12: 116.2 us, 4: 130.1, 16: 125.4), 4 for odd (N = 11: 129.8, 8: 152.3, 16: 177.8).
 constexpr int line_default_elements(int N) { return N <= 10 ? 16 : (N % 2 ? 4 : 8); }
 
 // From this order the line contraction is even-odd (dhat_even_odd): N = 8,
@@ -524,7 +534,7 @@ __global__ void __launch_bounds__(LineTile<N, R, E>::kThreads, LineTile<N, R, E>
     // n (w + wR) / 2. Ghost states as in stage_kernel.
     const auto side_flux = [&](int s, int idx, R op, R ou, R ov, R (&F)[3]) {
         // Keeps the loads of the contraction from being hoisted over the flux:
-        // N = 8 FP64 126 registers instead of 166 (3 tiles an SM instead of 2).
+        // N = 8 FP64 128 registers instead of 166 (3 tiles an SM instead of 2).
         asm volatile("" ::: "memory");
         const R nx = side[s * E + e], ny = side[4 * E + s * E + e], sf = side[8 * E + s * E + e];
         const int to = to_s[s * E + e];

@@ -172,8 +172,8 @@ __device__ __forceinline__ void cp_async8_stream(void* dst, const void* src, uin
 }
 // Programmatic dependent launch (PTX ISA: griddepcontrol). A kernel launched
 // by launch_dependent may start while the launch before it on the stream still
-// runs, once every CTA of that one has started (or called
-// pdl_launch_dependents). Before pdl_wait, which returns when the launches
+// runs, once every CTA of that one has called pdl_launch_dependents or exited.
+// Before pdl_wait, which returns when the launches
 // before it are complete and their writes visible, it touches only its own
 // shared memory and arrays that no launch of the run writes (the mesh plan).
 // The stage kernels let the next launch start late, when their new state is

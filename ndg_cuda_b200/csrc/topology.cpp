@@ -21,7 +21,6 @@
 #include <algorithm>
 #include <cmath>
 #include <fstream>
-#include <limits>
 #include <sstream>
 #include <unordered_map>
 
@@ -273,23 +272,24 @@ bool jacobians_regular(const SidePlan& plan, int64_t K, double t) {
     // x_xi and y_xi are linear in eta, x_eta and y_eta in xi, and so is J in each
     // of them: between its values at the four outermost nodes, and its terms
     // no larger than there.
+    const double near = 0.25 * (1.0 + t), far = 0.25 * (1.0 - t);
     for (int64_t e = 0; e < K; ++e) {
         const double* c = plan.corners.data() + 8 * e;
-        double least = std::numeric_limits<double>::infinity(), most = 0.0, terms = 0.0;
-        int signs = 0;
-        for (int corner = 0; corner < 4; ++corner) {
-            const double xi = corner & 1 ? t : -t, eta = corner & 2 ? t : -t;
-            const double x_xi = 0.25 * ((1.0 - eta) * (c[2] - c[0]) + (1.0 + eta) * (c[4] - c[6]));
-            const double y_xi = 0.25 * ((1.0 - eta) * (c[3] - c[1]) + (1.0 + eta) * (c[5] - c[7]));
-            const double x_eta = 0.25 * ((1.0 - xi) * (c[6] - c[0]) + (1.0 + xi) * (c[4] - c[2]));
-            const double y_eta = 0.25 * ((1.0 - xi) * (c[7] - c[1]) + (1.0 + xi) * (c[5] - c[3]));
-            const double J = x_xi * y_eta - x_eta * y_xi, a = std::abs(J);
-            signs += J > 0.0 ? 1 : (J < 0.0 ? -1 : 0);
-            least = std::min(least, a);
-            most = std::max(most, a);
-            terms = std::max(terms, std::abs(x_xi * y_eta) + std::abs(x_eta * y_xi));
-        }
-        if (!(std::abs(signs) == 4 && least >= 0x1p-1000 && most <= 0x1p1000 && least >= 1e-12 * terms)) return false;
+        const double ax = c[2] - c[0], ay = c[3] - c[1], bx = c[4] - c[6], by = c[5] - c[7];  // bottom and top edge
+        const double cx = c[6] - c[0], cy = c[7] - c[1], dx = c[4] - c[2], dy = c[5] - c[3];  // left and right edge
+        const double x_xi[2] = {near * ax + far * bx, far * ax + near * bx}, y_xi[2] = {near * ay + far * by, far * ay + near * by};
+        const double x_eta[2] = {near * cx + far * dx, far * cx + near * dx}, y_eta[2] = {near * cy + far * dy, far * cy + near * dy};
+        const double sign = x_xi[0] * y_eta[0] < x_eta[0] * y_xi[0] ? -1.0 : 1.0;
+        double least = 0x1p1000, terms = 0.0;
+        bool normal = true;  // false on a NaN too
+        for (int i = 0; i < 2; ++i)
+            for (int j = 0; j < 2; ++j) {
+                const double u = x_xi[j] * y_eta[i], v = x_eta[i] * y_xi[j], J = sign * (u - v);
+                normal = normal && J >= 0x1p-1000 && J <= 0x1p1000;
+                least = std::min(least, J);
+                terms = std::max(terms, std::abs(u) + std::abs(v));
+            }
+        if (!(normal && least >= 1e-12 * terms)) return false;
     }
     return true;
 }
