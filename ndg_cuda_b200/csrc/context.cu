@@ -1156,6 +1156,7 @@ ndg_status ndg_tables_build(ndg_ctx* ctx, int32_t N_max, int64_t n_interp) {
         ctx->has_tables = true;
         if (ctx->device >= 0) {
             check_cuda(dev::upload_tables(ctx->tables), "table upload");
+            check_cuda(dev::upload_general_tables(ctx->tables), "table upload");
             check_cuda(dev::upload_polynomials(ctx->tables), "table upload");
         }
     });

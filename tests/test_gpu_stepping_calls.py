@@ -271,3 +271,39 @@ def test_a_mixed_mesh_with_smaller_tiles_loaded_meanwhile_changes_nothing(mode, 
         results.append(_get(m))
         m.close()
     assert np.isfinite(results[0]).all() and np.array_equal(results[0], results[1])
+
+
+_TABLES_FIRST = """
+import sys
+import numpy as np
+import ndg_cuda_b200 as ndg
+from tests import meshgen
+
+if sys.argv[1] == "tables":
+    class Context(ndg._Context):
+        def __init__(self, *args):
+            super().__init__(*args)
+            assert ndg.lib().ndg_tables_build(self.h, 9, 2) == 0
+    ndg._Context = Context
+m = ndg.Mesh2D_t(meshgen.uniform_zone(8, boundary=meshgen.WALL), 4, maximum_N=8)
+m.initial_conditions()
+m.adapt((np.arange(64) % 2).astype(np.int32), np.full(64, 2.0))
+ndg.Solver2D_t.run(m, 3)
+np.save(sys.argv[2], np.concatenate([m.get_field(f) for f in "puv"]))
+"""
+
+
+def test_tables_built_before_the_mesh_serve_mixed_orders(tmp_path):
+    """ndg_tables_build, then a mesh in the same context, which uses those
+    tables and becomes a mixed-order one; in processes that load nothing else."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    out = []
+    for how in ("mesh", "tables"):
+        path = str(tmp_path / f"{how}.npy")
+        subprocess.run([sys.executable, "-c", _TABLES_FIRST, how, path], check=True, cwd=root, capture_output=True, text=True, timeout=300)
+        out.append(np.load(path))
+    assert np.isfinite(out[0]).all() and np.linalg.norm(out[0]) > 0
+    assert np.array_equal(out[0], out[1])
